@@ -7,14 +7,13 @@
 // (d0, d1) in ((1,0,s0), (0,1,s1), (1,1,hyp), (1,-1,hyp)), parity on the
 // axis-0 coordinate of endpoint a when d0 != 0, else on its axis-1 coordinate.
 //
-// relax_full_kernel      -- one full-domain iteration (8 colour sub-phases) per
-//                           launch with temporal blocking: a (T+2*8)^2 halo
-//                           box is TMA-loaded into shared memory, all eight
-//                           sub-phases run there (the exact region shrinks by
+// Full-domain sweeps (relax_critical_slope itself) are in sb_sweep.cuh.
+//
+// relax_reached_kernel   -- one reached-gated iteration per launch, temporally
+//                           blocked: a (T+2*8)^2 halo box in shared memory runs
+//                           all eight sub-phases (the exact region shrinks by
 //                           one cell per sub-phase), the T^2 interior is
-//                           written back; the iteration's max excess (over all
-//                           pairs of each sub-phase, before its update) feeds
-//                           the convergence test on the device.
+//                           written back.
 // frontier_*_kernel      -- production compact-frontier rounds
 //                           (runtime/v2_physics_core.py:1172-1254 over
 //                           solvers/warp_compact_frontier.py:56-130): the
@@ -72,162 +71,12 @@ __device__ __forceinline__ void dir_of(int d, int& d0, int& d1) {
 }
 
 // ------------------------------------------------------------------------
-// Full-domain relaxation (one iteration per launch).
-// ------------------------------------------------------------------------
-template <bool FX>
-__global__ void __launch_bounds__(kThreads)
-    relax_full_kernel(const RelaxConst c, const __grid_constant__ CUtensorMap tm0,
-                      const __grid_constant__ CUtensorMap tm1,
-                      typename FvTypes<FX>::H* __restrict__ f0,
-                      typename FvTypes<FX>::H* __restrict__ f1, RelaxControl* ctl,
-                      cudaGraphConditionalHandle handle, int use_handle) {
-  using H = typename FvTypes<FX>::H;
-  __shared__ alignas(128) H s[kRelaxBox * kRelaxBox];
-  __shared__ alignas(8) uint64_t bar;
-  __shared__ double red[kThreads / 32];
-  __shared__ int last;
-  if (*(volatile int*)&ctl->done) return;
-  const int parity_buf = ctl->parity;
-  const int t1 = blockIdx.x % c.tiles1, t0 = blockIdx.x / c.tiles1;
-  const int g0 = t0 * kRelaxTile - kRelaxHalo, g1 = t1 * kRelaxTile - kRelaxHalo;
-  if (threadIdx.x == 0) mbar_init(&bar, 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    mbar_expect_tx(&bar, kRelaxBox * kRelaxBox * (unsigned)sizeof(H));
-    tma_load_2d(s, parity_buf ? &tm1 : &tm0, g1, g0, &bar);
-  }
-  const bool loaded = mbar_wait(&bar, 0);
-  // a box wholly inside the domain needs no domain checks
-  const bool inner = g0 >= 0 && g1 >= 0 && g0 + kRelaxBox <= c.n0 && g1 + kRelaxBox <= c.n1;
-  double worst = 0.0;
-  for (int d = 0; d < 4; ++d) {
-    int d0, d1;
-    dir_of(d, d0, d1);
-    for (int par = 0; par < 2; ++par) {
-      // (1) max excess, before this sub-phase's update, over the pairs owned by
-      // the interior whose endpoint a has the inactive parity (those of the
-      // active parity are taken in (2) as they are read, before their update)
-      constexpr int kHalfTile = kRelaxTile / 2;
-      const int ifirst = d0 ? ((1 - par - g0) & 1) : ((1 - par - g1) & 1);
-      for (int k = threadIdx.x; k < kHalfTile * kRelaxTile; k += kThreads) {
-        const int la0 = kRelaxHalo + (d0 ? ifirst + 2 * (k / kRelaxTile) : k / kHalfTile);
-        const int la1 = kRelaxHalo + (d0 ? k % kRelaxTile : ifirst + 2 * (k % kHalfTile));
-        const int a0 = g0 + la0, a1 = g1 + la1, b0 = a0 + d0, b1 = a1 + d1;
-        if (a0 >= c.n0 || a1 >= c.n1 || b0 >= c.n0 || b1 < 0 || b1 >= c.n1) continue;
-        const int ia = la0 * kRelaxBox + la1, ib = (la0 + d0) * kRelaxBox + la1 + d1;
-        double ex;
-        if constexpr (FX) {
-          const long long df = (long long)s[ia] - (long long)s[ib];
-          ex = (double)(df < 0 ? -df : df) - c.crit_q[d];  // in quanta
-        } else {
-          ex = fmax(fabs(s[ia] - s[ib]) - c.crit[d], 0.0);
-        }
-        worst = fmax(worst, ex);
-      }
-      __syncthreads();
-      // (2) Jacobi update of the active-parity pairs inside the box: only the
-      // rows (d0 != 0) or columns (d0 == 0) whose global index has parity
-      // par hold an active endpoint a.  Sub-phase i (0-7) only needs pairs
-      // with endpoint a in [i, kRelaxBox - i) on both axes: every pair that
-      // touches a cell still exact after it (distance > i from the box edge)
-      // has a there, and its inputs are exact (distance >= i).
-      if (loaded) {
-        const int lo = d * 2 + par, hi = kRelaxBox - lo, span = hi - lo;
-        const int first = d0 ? ((par - g0) & 1) : ((par - g1) & 1);
-        const int start = lo + ((first - lo) & 1);  // first line of the parity in [lo, hi)
-        const int lines = (hi - start + 1) >> 1;
-        // k / ncol by a multiply and shift (exact for k < 2^20 / 48)
-        const int ncol = d0 ? span : lines;
-        const unsigned inv = ((1u << 20) + (unsigned)ncol - 1u) / (unsigned)ncol;
-        for (int k = threadIdx.x; k < lines * span; k += kThreads) {
-          const int q = (int)(((unsigned)k * inv) >> 20), rem = k - q * ncol;
-          int la0, la1;
-          if (d0) {
-            la0 = start + 2 * q;
-            la1 = lo + rem;
-          } else {
-            la0 = lo + q;
-            la1 = start + 2 * rem;
-          }
-          const int lb0 = la0 + d0, lb1 = la1 + d1;
-          if (lb0 >= kRelaxBox || lb1 < 0 || lb1 >= kRelaxBox) continue;
-          const int a0 = g0 + la0, a1 = g1 + la1, b0 = a0 + d0, b1 = a1 + d1;
-          if (!inner) {
-            if (a0 < 0 || a1 < 0 || a0 >= c.n0 || a1 >= c.n1) continue;
-            if (b0 >= c.n0 || b1 < 0 || b1 >= c.n1) continue;
-          }
-          const int ia = la0 * kRelaxBox + la1, ib = lb0 * kRelaxBox + lb1;
-          const bool owned = la0 >= kRelaxHalo && la0 < kRelaxHalo + kRelaxTile &&
-                             la1 >= kRelaxHalo && la1 < kRelaxHalo + kRelaxTile;
-          if constexpr (FX) {
-            const long long df = (long long)s[ia] - (long long)s[ib];
-            const double ex = (double)(df < 0 ? -df : df) - c.crit_q[d];
-            if (owned) worst = fmax(worst, ex);
-            if (ex > 0.0) {
-              const long long t = (long long)ceil(ex * 0.5);
-              const long long st = df < 0 ? -t : t;
-              s[ia] = (H)(s[ia] - st);
-              s[ib] = (H)(s[ib] + st);
-            }
-          } else {
-            const double diff = s[ia] - s[ib];
-            const double ex = fmax(fabs(diff) - c.crit[d], 0.0);
-            if (owned) worst = fmax(worst, ex);
-            const double sg = diff > 0.0 ? 1.0 : (diff < 0.0 ? -1.0 : 0.0);
-            const double t = 0.5 * ex * sg;
-            s[ia] = s[ia] - t;
-            s[ib] = s[ib] + t;
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  // write back the interior into the other buffer
-  H* dst = parity_buf ? f0 : f1;
-  for (int k = threadIdx.x; k < kRelaxTile * kRelaxTile; k += kThreads) {
-    const int la0 = kRelaxHalo + k / kRelaxTile, la1 = kRelaxHalo + k % kRelaxTile;
-    const int a0 = g0 + la0, a1 = g1 + la1;
-    if (a0 < c.n0 && a1 < c.n1 && loaded) dst[(size_t)a0 * c.pitch + a1] = s[la0 * kRelaxBox + la1];
-  }
-  worst = warp_max(worst);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = worst;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m = 0.0;
-    for (int w = 0; w < kThreads / 32; ++w) m = fmax(m, red[w]);
-    if (!loaded) atomicExch(&ctl->status, 6);
-    atomicMax(&ctl->max_excess_bits, (unsigned long long)__double_as_longlong(m));
-    __threadfence();
-    last = atomicAdd(&ctl->arrive, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last || threadIdx.x != 0) return;
-  __threadfence();
-  const double m = __longlong_as_double((long long)ctl->max_excess_bits);
-  ctl->arrive = 0;
-  ctl->max_excess_bits = 0;
-  ctl->iterations += 1;
-  ctl->parity = parity_buf ^ 1;
-  if (ctl->status) {
-    ctl->done = 1;
-  } else if (m <= (FX ? c.tol_q : c.tol)) {
-    ctl->converged = 1;
-    ctl->done = 1;
-  } else if (ctl->iterations >= c.max_iterations) {
-    ctl->done = 1;
-  }
-  __threadfence();
-  if (use_handle) cudaGraphSetConditional(handle, ctl->done ? 0u : 1u);
-}
-
-// ------------------------------------------------------------------------
 // Reached-gated full-domain iteration: the event-driven reached-bbox
 // MiniSlope backend (EventDrivenMinimumSlopeAdapter._relax_dynamic_frontier,
 // solvers/event_driven_slope.py:166-302).
 //
-// Same temporal blocking as relax_full_kernel (48^2 box, 8 sub-phases in
-// shared memory, 32^2 interior written back), plus the reached mask staged
+// A 48^2 TMA box, 8 sub-phases in shared memory, the 32^2 interior written
+// back, and the reached mask staged
 // in a second TMA box: a pair moves only if one endpoint is reached, both
 // endpoints of a moved pair become reached (the mask can spread one cell per
 // sub-phase, so the 8-cell halo stays exact), and the iteration maximum takes

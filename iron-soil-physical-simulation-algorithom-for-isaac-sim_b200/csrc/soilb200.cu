@@ -30,6 +30,7 @@
 #include "sb_ledger.cuh"
 #include "sb_labels.cuh"
 #include "sb_relax.cuh"
+#include "sb_sweep.cuh"
 #include "sb_exchange.cuh"
 #include "sb_deposition.cuh"
 #include "sb_avalanche.cuh"
@@ -173,10 +174,13 @@ struct sb_ctx {
   int frontier_grid = 1;  // CTAs of the list-driven frontier kernels
   RelaxControl* rctl = nullptr;
   RelaxControl* rctl_host = nullptr;
-  LoopGraph relax_full;
-  LoopGraph relax_full2;  // second cached relaxation graph (e.g. short sweeps vs. to tolerance)
+  // full-domain sweeps: loop control, per-tile change flags (two iterations),
+  // CTAs that fit the device at once
+  SweepControl* sweep = nullptr;
+  SweepControl* sweep_host = nullptr;
+  int* sweep_act = nullptr;
+  int sweep_ctas = 1;
   LoopGraph relax_reached;  // reached-gated (event-driven) sweep to tolerance
-  int relax_lru = 0;
   LoopGraph frontier;
   // fused plain-path step
   PathState* pstate = nullptr;
@@ -854,6 +858,20 @@ int sb_ctx_create(const sb_grid_desc* desc, sb_ctx** out) {
   SB_CUDA(ctx, cudaMalloc(&ctx->phase[0], nt * 4));
   SB_CUDA(ctx, cudaMalloc(&ctx->phase[1], nt * 4));
   SB_CUDA(ctx, cudaMemsetAsync(ctx->ftile_next, 0, nt * 4, ctx->stream));
+  {
+    const long long tiles = (long long)((d.nx + kSweepInner - 1) / kSweepInner) *
+                            ((d.ny + kSweepRows - 2 * kSweepHalo - 1) / (kSweepRows - 2 * kSweepHalo));
+    const void* fn = d.precision == SB_FX32 ? (const void*)sweep_kernel<true, kSweepRows>
+                                            : (const void*)sweep_kernel<false, kSweepRows>;
+    int per_sm = 0, sms = 0;
+    SB_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d.device));
+    SB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSweepThreads, 0));
+    ctx->sweep_ctas = std::max(1, per_sm * sms);
+    SB_CUDA(ctx, cudaMalloc(&ctx->sweep_act, (size_t)tiles * 2 * sizeof(int)));
+    SB_CUDA(ctx, cudaMalloc(&ctx->sweep, sizeof(SweepControl)));
+    SB_CUDA(ctx, cudaMemsetAsync(ctx->sweep, 0, sizeof(SweepControl), ctx->stream));
+    SB_CUDA(ctx, cudaMallocHost(&ctx->sweep_host, sizeof(SweepControl)));
+  }
   SB_CUDA(ctx, cudaMalloc(&ctx->rctl, sizeof(RelaxControl)));
   SB_CUDA(ctx, cudaMemsetAsync(ctx->rctl, 0, sizeof(RelaxControl), ctx->stream));
   SB_CUDA(ctx, cudaMallocHost(&ctx->rctl_host, sizeof(RelaxControl)));
@@ -935,8 +953,6 @@ int sb_ctx_destroy(sb_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->mobile.exec) cudaGraphExecDestroy(ctx->mobile.exec);
   if (ctx->mobile.graph) cudaGraphDestroy(ctx->mobile.graph);
-  ctx->relax_full.reset();
-  ctx->relax_full2.reset();
   ctx->relax_reached.reset();
   ctx->frontier.reset();
   void* ptrs[] = {ctx->b, ctx->z, ctx->h[0], ctx->h[1], ctx->qx[0], ctx->qx[1], ctx->qy[0],
@@ -948,7 +964,7 @@ int sb_ctx_destroy(sb_ctx* ctx) {
                   ctx->roots.area6, ctx->roots.volume, ctx->roots.exc_start, ctx->roots.exc_stop,
                   ctx->roots.max_exc_start, ctx->roots.max_exc_stop, ctx->roots.prev_overlap,
                   ctx->root_list, ctx->lout, ctx->b_alt, ctx->ftile_next, ctx->phase[0],
-                  ctx->phase[1], ctx->rctl, ctx->xidx, ctx->xval, ctx->xout, ctx->xpart, ctx->pstate,
+                  ctx->phase[1], ctx->rctl, ctx->sweep, ctx->sweep_act, ctx->xidx, ctx->xval, ctx->xout, ctx->xpart, ctx->pstate,
                   ctx->path_count, ctx->forcing, ctx->m2r, ctx->dep_out, ctx->owned_surface,
                   ctx->act_count, ctx->act_first, ctx->act_last, ctx->r2m, ctx->initial_b,
                   ctx->ptiles, ctx->mob_out, ctx->pers_out, ctx->surf_before, ctx->dtiles,
@@ -957,6 +973,7 @@ int sb_ctx_destroy(sb_ctx* ctx) {
     if (p) cudaFree(p);
   if (ctx->lout_host) cudaFreeHost(ctx->lout_host);
   if (ctx->rctl_host) cudaFreeHost(ctx->rctl_host);
+  if (ctx->sweep_host) cudaFreeHost(ctx->sweep_host);
   for (cudaEvent_t e : ctx->ev_loop)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->ev_path)
@@ -1444,152 +1461,70 @@ __global__ void relax_reset_kernel(RelaxControl* ctl) {
   }
 }
 
+// Constants of a full-domain relaxation and its cooperative launch: every CTA
+// resident, at most one warp per tile.
 template <bool FX>
-static int build_relax_full(sb_ctx* ctx, const RelaxConst& c, LoopGraph& lg) {
-  lg.reset();
-  cudaGraph_t g;
-  SB_CUDA(ctx, cudaGraphCreate(&g, 0));
-  lg.graph = g;
-  cudaGraphConditionalHandle handle;
-  SB_CUDA(ctx, cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault));
-  cudaGraphNode_t n_reset, n_loop, n_body;
-  {
-    void* args[] = {(void*)&ctx->rctl};
-    int rc = add_kernel(ctx, g, &n_reset, nullptr, 0, (void*)relax_reset_kernel, dim3(1), 0, args);
-    if (rc) return rc;
+static int launch_sweeps(sb_ctx* ctx, const RelaxConst& c) {
+  SweepConst k{};
+  k.n0 = c.n0;
+  k.n1 = c.n1;
+  k.pitch = c.pitch;
+  k.tiles1 = (c.n1 + kSweepInner - 1) / kSweepInner;
+  k.ntiles = k.tiles1 * ((c.n0 + kSweepRows - 2 * kSweepHalo - 1) / (kSweepRows - 2 * kSweepHalo));
+  k.max_iterations = c.max_iterations;
+  k.tol = c.tol;
+  for (int d = 0; d < 4; ++d) {
+    k.crit[d] = c.crit[d];
+    // a pair moves from the first whole difference above crit_q on, and is above
+    // the tolerance from the first one with (double)u - crit_q > tol_q on
+    const double crit = std::floor(c.crit_q[d]);
+    k.C[d] = crit >= 4294967295.0 ? 0xffffffffu : (unsigned)crit;
+    double u = std::floor(c.crit_q[d] + c.tol_q);
+    while (u > crit && u - c.crit_q[d] > c.tol_q) u -= 1.0;
+    while (u - c.crit_q[d] <= c.tol_q && u < 4294967296.0) u += 1.0;
+    const double thr = u - crit;
+    k.thr[d] = u >= 4294967296.0 ? 0xffffffffu : (unsigned)std::max(thr, 1.0);
   }
-  cudaGraphNodeParams cp{};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = handle;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  SB_CUDA(ctx, cudaGraphAddNode(&n_loop, g, &n_reset, 1, &cp));
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  RelaxConst cc = c;
-  int use_handle = 1;
-  const int tiles1 = (c.n1 + kRelaxTile - 1) / kRelaxTile;
-  const int tiles0 = (c.n0 + kRelaxTile - 1) / kRelaxTile;
-  RelaxConst ck = cc;
-  ck.tiles1 = tiles1;
-  void* args[] = {(void*)&ck, (void*)&ctx->tm_relax[0], (void*)&ctx->tm_relax[1],
-                  (void*)&ctx->b, (void*)&ctx->b_alt, (void*)&ctx->rctl, (void*)&handle,
-                  (void*)&use_handle};
-  int rc = add_kernel(ctx, body, &n_body, nullptr, 0, (void*)relax_full_kernel<FX>,
-                      dim3(tiles0 * tiles1), 0, args);
-  if (rc) return rc;
-  // leave the result in b_eff whichever ping-pong buffer it ended in
-  cudaGraphNode_t n_copy, n_par;
-  {
-    long long count = (long long)ctx->pitch * ctx->d.ny;
-    void* cargs[] = {(void*)&ctx->b_alt, (void*)&ctx->b, (void*)&count, (void*)&ctx->rctl};
-    if ((rc = add_kernel(ctx, g, &n_copy, &n_loop, 1, (void*)relax_copyback_kernel<FX>,
-                         dim3(grid_for(count)), 0, cargs)))
-      return rc;
-    void* pargs[] = {(void*)&ctx->rctl};
-    if ((rc = add_kernel(ctx, g, &n_par, &n_copy, 1, (void*)relax_parity_clear_kernel, dim3(1), 0,
-                         pargs)))
-      return rc;
-  }
-  SB_CUDA(ctx, cudaGraphInstantiate(&lg.exec, g, 0));
-  lg.key = c;
-  lg.valid = true;
+  const int per = kSweepThreads / 32;
+  const int grid = std::min((k.ntiles + per - 1) / per, ctx->sweep_ctas);
+  typename FvTypes<FX>::H *f0 = (typename FvTypes<FX>::H*)ctx->b,
+                          *f1 = (typename FvTypes<FX>::H*)ctx->b_alt;
+  int *a0 = ctx->sweep_act, *a1 = ctx->sweep_act + k.ntiles;
+  void* args[] = {(void*)&k, (void*)&f0, (void*)&f1, (void*)&a0, (void*)&a1, (void*)&ctx->sweep};
+  SB_CUDA(ctx, cudaLaunchCooperativeKernel((void*)sweep_kernel<FX, kSweepRows>, dim3(grid),
+                                           dim3(kSweepThreads), args, 0, ctx->stream));
+  ctx->launches++;
   return SB_OK;
 }
 
-// Cached graph for these parameters (two slots, least recently used replaced).
-static int relax_graph_for(sb_ctx* ctx, const RelaxConst& c, LoopGraph** out) {
-  LoopGraph* slots[2] = {&ctx->relax_full, &ctx->relax_full2};
-  for (int i = 0; i < 2; ++i)
-    if (slots[i]->valid && std::memcmp(&slots[i]->key, &c, sizeof(RelaxConst)) == 0) {
-      ctx->relax_lru = i ^ 1;
-      *out = slots[i];
-      return SB_OK;
-    }
-  const int victim = ctx->relax_lru;
-  const int rc = fx(ctx) ? build_relax_full<true>(ctx, c, *slots[victim])
-                         : build_relax_full<false>(ctx, c, *slots[victim]);
+static int relax_full(sb_ctx* ctx, const sb_relax_params* p) {
+  RelaxConst c;
+  int rc = relax_const(ctx, p, &c, kRelaxTile);
   if (rc) return rc;
-  ctx->relax_lru = victim ^ 1;
-  *out = slots[victim];
-  return SB_OK;
-}
-
-// SOILB200_NO_GRAPH=1 (profilers that cannot see kernel nodes of a graph
-// with conditional nodes): the sweep graph's kernels launched from the host,
-// the loop flag read back after every sweep.
-template <bool FX>
-static int relax_full_host_loop(sb_ctx* ctx, const RelaxConst& c) {
-  void* rargs[] = {(void*)&ctx->rctl};
-  SB_CUDA(ctx, cudaLaunchKernel((void*)relax_reset_kernel, dim3(1), dim3(kThreads), rargs, 0,
-                                ctx->stream));
-  RelaxConst ck = c;
-  ck.tiles1 = (c.n1 + kRelaxTile - 1) / kRelaxTile;
-  const int tiles0 = (c.n0 + kRelaxTile - 1) / kRelaxTile;
-  cudaGraphConditionalHandle handle{};
-  int no_handle = 0;
-  void* args[] = {(void*)&ck, (void*)&ctx->tm_relax[0], (void*)&ctx->tm_relax[1],
-                  (void*)&ctx->b, (void*)&ctx->b_alt, (void*)&ctx->rctl, (void*)&handle,
-                  (void*)&no_handle};
-  for (long long it = 0; it <= (long long)c.max_iterations; ++it) {
-    SB_CUDA(ctx, cudaLaunchKernel((void*)relax_full_kernel<FX>, dim3(tiles0 * ck.tiles1),
-                                  dim3(kThreads), args, 0, ctx->stream));
-    SB_CUDA(ctx, cudaMemcpyAsync(ctx->rctl_host, ctx->rctl, sizeof(RelaxControl),
-                                 cudaMemcpyDeviceToHost, ctx->stream));
-    SB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->rctl_host->done) break;
-  }
-  long long count = (long long)ctx->pitch * ctx->d.ny;
-  void* cargs[] = {(void*)&ctx->b_alt, (void*)&ctx->b, (void*)&count, (void*)&ctx->rctl};
-  SB_CUDA(ctx, cudaLaunchKernel((void*)relax_copyback_kernel<FX>, dim3(grid_for(count)),
-                                dim3(kThreads), cargs, 0, ctx->stream));
-  SB_CUDA(ctx, cudaLaunchKernel((void*)relax_parity_clear_kernel, dim3(1), dim3(kThreads), rargs,
-                                0, ctx->stream));
-  return SB_OK;
+  return fx(ctx) ? launch_sweeps<true>(ctx, c) : launch_sweeps<false>(ctx, c);
 }
 
 // Queues max_iterations (or fewer, if converged) sweeps without waiting for
 // them or reading their statistics back.
 extern "C" int sb_relax_sweeps(sb_ctx* ctx, const sb_relax_params* p) {
   if (!ctx || !p) return SB_ERR_BAD_ARG;
-  RelaxConst c;
-  int rc = relax_const(ctx, p, &c, kRelaxTile);
-  if (rc) return rc;
-  if (!ctx->use_graphs) {
-    rc = fx(ctx) ? relax_full_host_loop<true>(ctx, c) : relax_full_host_loop<false>(ctx, c);
-    ctx->launches += 3 + ctx->rctl_host->iterations;
-    return rc;
-  }
-  LoopGraph* lg = nullptr;
-  if ((rc = relax_graph_for(ctx, c, &lg))) return rc;
-  SB_CUDA(ctx, cudaGraphLaunch(lg->exec, ctx->stream));
-  ctx->launches += 3;
-  return SB_OK;
+  return relax_full(ctx, p);
 }
 
 extern "C" int sb_relax_full(sb_ctx* ctx, const sb_relax_params* p, sb_relax_stats* out) {
   if (!ctx || !p || !out) return SB_ERR_BAD_ARG;
-  RelaxConst c;
-  int rc = relax_const(ctx, p, &c, kRelaxTile);
+  int rc = relax_full(ctx, p);
   if (rc) return rc;
-  if (!ctx->use_graphs) {
-    rc = fx(ctx) ? relax_full_host_loop<true>(ctx, c) : relax_full_host_loop<false>(ctx, c);
-    if (rc) return rc;
-  } else {
-    LoopGraph* lg = nullptr;
-    if ((rc = relax_graph_for(ctx, c, &lg))) return rc;
-    SB_CUDA(ctx, cudaGraphLaunch(lg->exec, ctx->stream));
-  }
-  SB_CUDA(ctx, cudaMemcpyAsync(ctx->rctl_host, ctx->rctl, sizeof(RelaxControl),
+  SB_CUDA(ctx, cudaMemcpyAsync(ctx->sweep_host, ctx->sweep, sizeof(SweepControl),
                                cudaMemcpyDeviceToHost, ctx->stream));
   SB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  const RelaxControl& k = *ctx->rctl_host;
-  ctx->launches += 3 + k.iterations;
+  const SweepControl& k = *ctx->sweep_host;
   std::memset(out, 0, sizeof(*out));
   out->iterations = k.iterations;
   out->converged = k.converged;
   out->status = k.status;
   if (k.status == SB_ERR_WAIT_LIMIT)
-    return fail(ctx, SB_ERR_WAIT_LIMIT, "[soilb200] a bounded device wait gave up (TMA tile load)");
+    return fail(ctx, SB_ERR_WAIT_LIMIT, "[soilb200] a bounded device wait gave up (sweep barrier)");
   return SB_OK;
 }
 
