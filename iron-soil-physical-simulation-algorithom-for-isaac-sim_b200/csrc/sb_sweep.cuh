@@ -16,18 +16,18 @@
 // across lanes cost two shuffles; there is no shared memory and no block
 // barrier, and parities are compile-time because box origins are even.
 //
-// What bounds it: integer issue.  A pair is 8 integer operations (difference,
-// clamp to +-C, excess, half of it towards zero, the two new heights, the two
-// running extremes); the shared-memory kernel it replaces spent about 40 on
-// index arithmetic, 64-bit differences and double conversions, plus 16 block
-// barriers per iteration.  FX, every tile moving: 8.7 us per sweep at 701^2,
-// 34 us at 2048^2, 108 us at 4096^2; a cut pile settling: 7.1 us per sweep at
-// 701^2 (24 before), 9.7 at 2048^2 (135 before; 498 sweeps 64 -> 4.8 ms), 18
-// at 4096^2.  FP64 at 701^2: 12.4 us.  At 701^2 a sweep is latency: flags and
-// box from L2, 2.2 k instructions of one warp, the barrier.
-//
-// 32 box rows: 24 or 48 leave the chip emptier or redo more halo; with 32 a
-// 701^2 grid has 660 boxes, about one for each warp scheduler.
+// What bounds it: integer issue and instruction fetch (straight-line code; ncu
+// with 48 rows: 2.8 of 6.9 cycles per instruction wait for instructions).  A
+// pair is 8 integer operations (difference, clamp to +-C, excess, half of it
+// towards zero, the two new heights, the two running extremes); the
+// shared-memory kernel it replaces spent about 40 on index arithmetic, 64-bit
+// differences and double conversions, plus 16 block barriers per iteration.
+// FX, every tile moving, 24 rows: 7.8 us per sweep at 701^2, 32 at 2048^2; a cut
+// pile settling: 4.9 at 701^2 (24 before), 9.2 at 2048^2 (135 before), 19 at
+// 4096^2.  On small grids a sweep is latency: flags and box from L2, one warp's
+// instructions, the barrier.  A strip streamed through an 11-row register
+// window (no row halo, small code) was slower at every size: its chain of
+// sub-phases needs more instructions per cell than a box's shrinking rows.
 //
 // Tiles at rest are skipped: a box without any transfer in an iteration is the
 // same before the next one, so its tile runs again only after a tile of its
@@ -47,7 +47,8 @@ namespace sb {
 constexpr int kSweepHalo = 8;
 constexpr int kSweepCols = 64;                            // box columns of a warp
 constexpr int kSweepInner = kSweepCols - 2 * kSweepHalo;  // columns written back
-constexpr int kSweepRows = 32;                            // box rows
+// Box rows; relax_full chooses.
+constexpr int kSweepRows = 24, kSweepRowsTall = 48;
 constexpr int kSweepThreads = 128;
 constexpr unsigned kSweepPolls = 1u << 22;
 
@@ -299,7 +300,7 @@ __device__ __forceinline__ void sweep_box(const SweepConst& c, typename SweepOp<
 }
 
 template <bool FX, int R>
-__global__ void __launch_bounds__(kSweepThreads, FX ? 4 : 2)
+__global__ void __launch_bounds__(kSweepThreads, !FX ? 2 : R > 32 ? 3 : 4)
     sweep_kernel(const SweepConst c, typename FvTypes<FX>::H* f0, typename FvTypes<FX>::H* f1,
                  int* act0, int* act1, SweepControl* ctl) {
   using H = typename FvTypes<FX>::H;

@@ -92,10 +92,32 @@ struct LoopGraph {  // graph whose key is a RelaxConst
   }
 };
 
+// Buffers of one context collected first and placed in a single allocation
+// afterwards: about 70 cudaMalloc and 12 pinned allocations, and their release,
+// took 19 + 13 ms of a one-shot call (relax_critical_slope at 701^2).
+struct Arena {
+  struct Item {
+    void** p;
+    size_t offset;
+  };
+  std::vector<Item> items;
+  size_t bytes = 0;
+  template <typename T>
+  void add(T** p, size_t n) {
+    items.push_back({reinterpret_cast<void**>(p), bytes});
+    bytes += (n + 511) / 512 * 512;  // cudaMalloc's alignment
+  }
+  void place(void* base) {
+    for (const Item& i : items) *i.p = static_cast<char*>(base) + i.offset;
+  }
+};
+
 }  // namespace
 
 struct sb_ctx {
   sb_grid_desc d{};
+  void* arena = nullptr;       // every fixed-size device buffer below, one allocation
+  void* host_arena = nullptr;  // every pinned, mapped host record below
   int pitch = 0;        // elements per row
   size_t esize = 0;     // bytes per element of float-like fields
   cudaStream_t stream = nullptr;
@@ -174,12 +196,11 @@ struct sb_ctx {
   int frontier_grid = 1;  // CTAs of the list-driven frontier kernels
   RelaxControl* rctl = nullptr;
   RelaxControl* rctl_host = nullptr;
-  // full-domain sweeps: loop control, per-tile change flags (two iterations),
-  // CTAs that fit the device at once
+  // full-domain sweeps: loop control, per-tile change flags (two iterations)
   SweepControl* sweep = nullptr;
   SweepControl* sweep_host = nullptr;
   int* sweep_act = nullptr;
-  int sweep_ctas = 1;
+  int sms = 1;
   LoopGraph relax_reached;  // reached-gated (event-driven) sweep to tolerance
   LoopGraph frontier;
   // fused plain-path step
@@ -714,18 +735,13 @@ int sb_ctx_create(const sb_grid_desc* desc, sb_ctx** out) {
   const size_t field_bytes = (size_t)ctx->pitch * d.ny * ctx->esize;
   void** all[] = {&ctx->b, &ctx->z, &ctx->h[0], &ctx->h[1], &ctx->qx[0],
                   &ctx->qx[1], &ctx->qy[0], &ctx->qy[1], &ctx->ext_x, &ctx->ext_y};
-  for (void** p : all) {
-    SB_CUDA(ctx, cudaMalloc(p, field_bytes));
-    SB_CUDA(ctx, cudaMemsetAsync(*p, 0, field_bytes, ctx->stream));
-  }
-  SB_CUDA(ctx, cudaMalloc(&ctx->reached, (size_t)ctx->pitch * d.ny * sizeof(int32_t)));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->reached, 0, (size_t)ctx->pitch * d.ny * 4, ctx->stream));
-  SB_CUDA(ctx, cudaMalloc(&ctx->staging, (size_t)d.ny * d.nx * sizeof(double)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->range_error, sizeof(int)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->ctl, sizeof(FvControl)));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->ctl, 0, sizeof(FvControl), ctx->stream));
-  SB_CUDA(ctx, cudaMalloc(&ctx->io, sizeof(StepIO)));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->io, 0, sizeof(StepIO), ctx->stream));
+  Arena dev, host;
+  for (void** p : all) dev.add(p, field_bytes);
+  dev.add(&ctx->reached, (size_t)ctx->pitch * d.ny * sizeof(int32_t));
+  dev.add(&ctx->staging, (size_t)d.ny * d.nx * sizeof(double));
+  dev.add(&ctx->range_error, sizeof(int));
+  dev.add(&ctx->ctl, sizeof(FvControl));
+  dev.add(&ctx->io, sizeof(StepIO));
   const int tiles = ((d.nx + kTileX - 1) / kTileX) * ((d.ny + kTileY - 1) / kTileY);
   ctx->fv_blocks = tiles;
   if (d.precision == SB_FX32) {
@@ -766,21 +782,19 @@ int sb_ctx_create(const sb_grid_desc* desc, sb_ctx** out) {
   ctx->ledger_blocks = std::min(grid_for((long long)d.ny * d.nx), 3 * 148);
   const size_t np = (size_t)std::max({tiles, ctx->ledger_blocks, ctx->fv_stream_blocks}) *
                     (kFvPartial > L_NP ? kFvPartial : L_NP);
-  SB_CUDA(ctx, cudaMalloc(&ctx->partials, np * sizeof(double)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->ipartials, (size_t)ctx->ledger_blocks * kLedgerI64 * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->lpart_before, (size_t)ctx->ledger_blocks * L_NP * sizeof(double)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->lipart_before, (size_t)ctx->ledger_blocks * kLedgerI64 * 8));
+  dev.add(&ctx->partials, np * sizeof(double));
+  dev.add(&ctx->ipartials, (size_t)ctx->ledger_blocks * kLedgerI64 * 8);
+  dev.add(&ctx->lpart_before, (size_t)ctx->ledger_blocks * L_NP * sizeof(double));
+  dev.add(&ctx->lipart_before, (size_t)ctx->ledger_blocks * kLedgerI64 * 8);
   {
     const size_t nd = (size_t)kFvDiag * std::max(tiles, ctx->fv_stream_blocks);
-    SB_CUDA(ctx, cudaMalloc(&ctx->fv_diag, nd * sizeof(double)));
-    SB_CUDA(ctx, cudaMemsetAsync(ctx->fv_diag, 0, nd * sizeof(double), ctx->stream));
+    dev.add(&ctx->fv_diag, nd * sizeof(double));
   }
-  SB_CUDA(ctx, cudaMalloc(&ctx->arrive, sizeof(unsigned)));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->arrive, 0, sizeof(unsigned), ctx->stream));
-  SB_CUDA(ctx, cudaMalloc(&ctx->dt_dev, sizeof(double)));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->dt_host, sizeof(double)));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->ctl_host, sizeof(FvControl)));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->io_host, sizeof(StepIO)));
+  dev.add(&ctx->arrive, sizeof(unsigned));
+  dev.add(&ctx->dt_dev, sizeof(double));
+  host.add(&ctx->dt_host, sizeof(double));
+  host.add(&ctx->ctl_host, sizeof(FvControl));
+  host.add(&ctx->io_host, sizeof(StepIO));
   SB_CUDA(ctx, cudaEventCreate(&ctx->ev_loop[0]));
   SB_CUDA(ctx, cudaEventCreate(&ctx->ev_loop[1]));
   SB_CUDA(ctx, cudaEventCreate(&ctx->ev_path[0]));
@@ -793,54 +807,41 @@ int sb_ctx_create(const sb_grid_desc* desc, sb_ctx** out) {
   }
   // labelling buffers (flat ny*nx)
   const size_t n = (size_t)d.ny * d.nx;
-  SB_CUDA(ctx, cudaMalloc(&ctx->parent, n * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->slope, n * ctx->esize));
-  SB_CUDA(ctx, cudaMalloc(&ctx->severity, n * ctx->esize));
-  SB_CUDA(ctx, cudaMalloc(&ctx->latch, n * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->previous, n * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->export_cum, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->export_base, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->roots.count, n * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->roots.area6, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->roots.volume, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->roots.exc_start, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->roots.exc_stop, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->roots.max_exc_start, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->roots.max_exc_stop, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->roots.prev_overlap, n * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->root_list, n * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->lout, sizeof(LabelOut)));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->lout_host, sizeof(LabelOut)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->forcing, n * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->m2r, n * 8));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->forcing, 0, n * 4, ctx->stream));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->m2r, 0, n * 8, ctx->stream));
-  SB_CUDA(ctx, cudaMalloc(&ctx->surf_before, n * 8));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->surf_before, 0, n * 8, ctx->stream));
-  SB_CUDA(ctx, cudaMalloc(&ctx->owned_surface, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->act_count, n * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->act_first, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->act_last, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->r2m, n * 8));
-  {
-    void* hist[] = {ctx->owned_surface, ctx->act_first, ctx->act_last, ctx->r2m};
-    for (void* p : hist) SB_CUDA(ctx, cudaMemsetAsync(p, 0, n * 8, ctx->stream));
-    SB_CUDA(ctx, cudaMemsetAsync(ctx->act_count, 0, n * 4, ctx->stream));
-  }
-  SB_CUDA(ctx, cudaMalloc(&ctx->initial_b, (size_t)ctx->pitch * d.ny * ctx->esize));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->initial_b, 0, (size_t)ctx->pitch * d.ny * ctx->esize, ctx->stream));
-  SB_CUDA(ctx, cudaMalloc(&ctx->mob_out, sizeof(MobilizeOut)));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->mob_out_host, sizeof(MobilizeOut)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->pers_out, kPersistSlots * sizeof(double)));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->pers_out_host, kPersistSlots * sizeof(double)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->dep_out, sizeof(DepositionOut)));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->dep_out_host, sizeof(DepositionOut)));
-  void* zero_init[] = {ctx->parent, ctx->latch, ctx->previous, ctx->export_cum, ctx->export_base};
-  size_t zero_size[] = {n * 4, n * 4, n * 4, n * 8, n * 8};
-  for (int k = 0; k < 5; ++k) SB_CUDA(ctx, cudaMemsetAsync(zero_init[k], 0, zero_size[k], ctx->stream));
+  dev.add(&ctx->parent, n * 4);
+  dev.add(&ctx->slope, n * ctx->esize);
+  dev.add(&ctx->severity, n * ctx->esize);
+  dev.add(&ctx->latch, n * 4);
+  dev.add(&ctx->previous, n * 4);
+  dev.add(&ctx->export_cum, n * 8);
+  dev.add(&ctx->export_base, n * 8);
+  dev.add(&ctx->roots.count, n * 4);
+  dev.add(&ctx->roots.area6, n * 8);
+  dev.add(&ctx->roots.volume, n * 8);
+  dev.add(&ctx->roots.exc_start, n * 8);
+  dev.add(&ctx->roots.exc_stop, n * 8);
+  dev.add(&ctx->roots.max_exc_start, n * 8);
+  dev.add(&ctx->roots.max_exc_stop, n * 8);
+  dev.add(&ctx->roots.prev_overlap, n * 4);
+  dev.add(&ctx->root_list, n * 4);
+  dev.add(&ctx->lout, sizeof(LabelOut));
+  host.add(&ctx->lout_host, sizeof(LabelOut));
+  dev.add(&ctx->forcing, n * 4);
+  dev.add(&ctx->m2r, n * 8);
+  dev.add(&ctx->surf_before, n * 8);
+  dev.add(&ctx->owned_surface, n * 8);
+  dev.add(&ctx->act_count, n * 4);
+  dev.add(&ctx->act_first, n * 8);
+  dev.add(&ctx->act_last, n * 8);
+  dev.add(&ctx->r2m, n * 8);
+  dev.add(&ctx->initial_b, field_bytes);
+  dev.add(&ctx->mob_out, sizeof(MobilizeOut));
+  host.add(&ctx->mob_out_host, sizeof(MobilizeOut));
+  dev.add(&ctx->pers_out, kPersistSlots * sizeof(double));
+  host.add(&ctx->pers_out_host, kPersistSlots * sizeof(double));
+  dev.add(&ctx->dep_out, sizeof(DepositionOut));
+  host.add(&ctx->dep_out_host, sizeof(DepositionOut));
   // relaxation buffers
-  SB_CUDA(ctx, cudaMalloc(&ctx->b_alt, field_bytes));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->b_alt, 0, field_bytes, ctx->stream));
+  dev.add(&ctx->b_alt, field_bytes);
   ctx->ftiles0 = (d.ny + d.tile_size - 1) / d.tile_size;
   ctx->ftiles1 = (d.nx + d.tile_size - 1) / d.tile_size;
   {
@@ -852,42 +853,40 @@ int sb_ctx_create(const sb_grid_desc* desc, sb_ctx** out) {
         (int)std::min<long long>((long long)ctx->ftiles0 * ctx->ftiles1, 8LL * std::max(sms, 1));
   }
   const size_t nt = (size_t)ctx->ftiles0 * ctx->ftiles1;
-  SB_CUDA(ctx, cudaMalloc(&ctx->ptiles, nt * sizeof(int)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->dtiles, nt * sizeof(int)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->ftile_next, nt * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->phase[0], nt * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->phase[1], nt * 4));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->ftile_next, 0, nt * 4, ctx->stream));
+  dev.add(&ctx->ptiles, nt * sizeof(int));
+  dev.add(&ctx->dtiles, nt * sizeof(int));
+  dev.add(&ctx->ftile_next, nt * 4);
+  dev.add(&ctx->phase[0], nt * 4);
+  dev.add(&ctx->phase[1], nt * 4);
   {
-    const long long tiles = (long long)((d.nx + kSweepInner - 1) / kSweepInner) *
-                            ((d.ny + kSweepRows - 2 * kSweepHalo - 1) / (kSweepRows - 2 * kSweepHalo));
-    const void* fn = d.precision == SB_FX32 ? (const void*)sweep_kernel<true, kSweepRows>
-                                            : (const void*)sweep_kernel<false, kSweepRows>;
-    int per_sm = 0, sms = 0;
-    SB_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d.device));
-    SB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSweepThreads, 0));
-    ctx->sweep_ctas = std::max(1, per_sm * sms);
-    SB_CUDA(ctx, cudaMalloc(&ctx->sweep_act, (size_t)tiles * 2 * sizeof(int)));
-    SB_CUDA(ctx, cudaMalloc(&ctx->sweep, sizeof(SweepControl)));
-    SB_CUDA(ctx, cudaMemsetAsync(ctx->sweep, 0, sizeof(SweepControl), ctx->stream));
-    SB_CUDA(ctx, cudaMallocHost(&ctx->sweep_host, sizeof(SweepControl)));
+    SB_CUDA(ctx, cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, d.device));
+    const int inner = kSweepRows - 2 * kSweepHalo;
+    const size_t tiles =
+        (size_t)((d.nx + kSweepInner - 1) / kSweepInner) * ((d.ny + inner - 1) / inner);
+    dev.add(&ctx->sweep_act, tiles * 2 * sizeof(int));
+    dev.add(&ctx->sweep, sizeof(SweepControl));
+    host.add(&ctx->sweep_host, sizeof(SweepControl));
   }
-  SB_CUDA(ctx, cudaMalloc(&ctx->rctl, sizeof(RelaxControl)));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->rctl, 0, sizeof(RelaxControl), ctx->stream));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->rctl_host, sizeof(RelaxControl)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->xidx, n * 4));
-  SB_CUDA(ctx, cudaMalloc(&ctx->xval, n * 8));
-  SB_CUDA(ctx, cudaMalloc(&ctx->xout, sizeof(ExchangeOut)));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->xout, 0, sizeof(ExchangeOut), ctx->stream));  // arrive = 0
+  dev.add(&ctx->rctl, sizeof(RelaxControl));
+  host.add(&ctx->rctl_host, sizeof(RelaxControl));
+  dev.add(&ctx->xidx, n * 4);
+  dev.add(&ctx->xval, n * 8);
+  dev.add(&ctx->xout, sizeof(ExchangeOut));
   static_assert(offsetof(ExchangeOut, momentum_w) == offsetof(ExchangeOut, volume_w_fp64) + 8,
                 "exchange_fold writes volume and momentum sums as one array");
-  SB_CUDA(ctx, cudaMalloc(&ctx->xpart, 3 * 148 * 8 * sizeof(double)));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->xout_host, sizeof(ExchangeOut)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->pstate, sizeof(PathState)));
-  SB_CUDA(ctx, cudaMemsetAsync(ctx->pstate, 0, sizeof(PathState), ctx->stream));
-  SB_CUDA(ctx, cudaMallocHost(&ctx->pstate_host, sizeof(PathState)));
-  SB_CUDA(ctx, cudaMalloc(&ctx->path_count, sizeof(int)));
-  SB_CUDA(ctx, cudaHostAlloc(&ctx->path_in, sizeof(PathInput), cudaHostAllocMapped));
+  dev.add(&ctx->xpart, 3 * 148 * 8 * sizeof(double));
+  host.add(&ctx->xout_host, sizeof(ExchangeOut));
+  dev.add(&ctx->pstate, sizeof(PathState));
+  host.add(&ctx->pstate_host, sizeof(PathState));
+  dev.add(&ctx->path_count, sizeof(int));
+  host.add(&ctx->path_in, sizeof(PathInput));
+  dev.add(&ctx->reached_alt, (size_t)ctx->pitch * d.ny * sizeof(int32_t));
+  SB_CUDA(ctx, cudaMalloc(&ctx->arena, dev.bytes));
+  dev.place(ctx->arena);
+  SB_CUDA(ctx, cudaMemsetAsync(ctx->arena, 0, dev.bytes, ctx->stream));
+  SB_CUDA(ctx, cudaHostAlloc(&ctx->host_arena, host.bytes, cudaHostAllocMapped));
+  host.place(ctx->host_arena);
+  std::memset(ctx->host_arena, 0, host.bytes);
   // TMA descriptors (box = halo tile of the FV kernel)
   int rc;
   {
@@ -897,9 +896,7 @@ int sb_ctx_create(const sb_grid_desc* desc, sb_ctx** out) {
       return rc;
     if ((rc = encode_2d(ctx, &ctx->tm_relax[1], ctx->b_alt, dt, ctx->esize, kRelaxBox, kRelaxBox)))
       return rc;
-    SB_CUDA(ctx, cudaMalloc(&ctx->reached_alt, (size_t)ctx->pitch * d.ny * sizeof(int32_t)));
-    SB_CUDA(ctx, cudaMemsetAsync(ctx->reached_alt, 0, (size_t)ctx->pitch * d.ny * 4, ctx->stream));
-    if ((rc = encode_2d(ctx, &ctx->tm_reached[0], ctx->reached, CU_TENSOR_MAP_DATA_TYPE_INT32, 4,
+      if ((rc = encode_2d(ctx, &ctx->tm_reached[0], ctx->reached, CU_TENSOR_MAP_DATA_TYPE_INT32, 4,
                         kRelaxBox, kRelaxBox)))
       return rc;
     if ((rc = encode_2d(ctx, &ctx->tm_reached[1], ctx->reached_alt, CU_TENSOR_MAP_DATA_TYPE_INT32,
@@ -955,44 +952,20 @@ int sb_ctx_destroy(sb_ctx* ctx) {
   if (ctx->mobile.graph) cudaGraphDestroy(ctx->mobile.graph);
   ctx->relax_reached.reset();
   ctx->frontier.reset();
-  void* ptrs[] = {ctx->b, ctx->z, ctx->h[0], ctx->h[1], ctx->qx[0], ctx->qx[1], ctx->qy[0],
-                  ctx->qy[1], ctx->ext_x, ctx->ext_y, ctx->reached, ctx->staging,
-                  ctx->range_error, ctx->ctl, ctx->io, ctx->partials, ctx->ipartials, ctx->fv_diag,
-                  ctx->lpart_before, ctx->lipart_before,
-                  ctx->arrive, ctx->dt_dev, ctx->parent, ctx->slope, ctx->severity, ctx->latch,
-                  ctx->previous, ctx->export_cum, ctx->export_base, ctx->roots.count,
-                  ctx->roots.area6, ctx->roots.volume, ctx->roots.exc_start, ctx->roots.exc_stop,
-                  ctx->roots.max_exc_start, ctx->roots.max_exc_stop, ctx->roots.prev_overlap,
-                  ctx->root_list, ctx->lout, ctx->b_alt, ctx->ftile_next, ctx->phase[0],
-                  ctx->phase[1], ctx->rctl, ctx->sweep, ctx->sweep_act, ctx->xidx, ctx->xval, ctx->xout, ctx->xpart, ctx->pstate,
-                  ctx->path_count, ctx->forcing, ctx->m2r, ctx->dep_out, ctx->owned_surface,
-                  ctx->act_count, ctx->act_first, ctx->act_last, ctx->r2m, ctx->initial_b,
-                  ctx->ptiles, ctx->mob_out, ctx->pers_out, ctx->surf_before, ctx->dtiles,
-                  ctx->q_rows, ctx->q_cols, ctx->q_out, ctx->reached_alt};
+  void* ptrs[] = {ctx->arena, ctx->q_rows, ctx->q_cols, ctx->q_out};
   for (void* p : ptrs)
     if (p) cudaFree(p);
-  if (ctx->lout_host) cudaFreeHost(ctx->lout_host);
-  if (ctx->rctl_host) cudaFreeHost(ctx->rctl_host);
-  if (ctx->sweep_host) cudaFreeHost(ctx->sweep_host);
   for (cudaEvent_t e : ctx->ev_loop)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->ev_path)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->ev_stage)
     if (e) cudaEventDestroy(e);
-  if (ctx->xout_host) cudaFreeHost(ctx->xout_host);
-  if (ctx->dep_out_host) cudaFreeHost(ctx->dep_out_host);
-  if (ctx->mob_out_host) cudaFreeHost(ctx->mob_out_host);
-  if (ctx->pers_out_host) cudaFreeHost(ctx->pers_out_host);
-  if (ctx->pstate_host) cudaFreeHost(ctx->pstate_host);
-  if (ctx->path_in) cudaFreeHost(ctx->path_in);
+  if (ctx->host_arena) cudaFreeHost(ctx->host_arena);
   if (ctx->path_idx) cudaFreeHost(ctx->path_idx);
   if (ctx->path_val) cudaFreeHost(ctx->path_val);
   if (ctx->path_exec) cudaGraphExecDestroy(ctx->path_exec);
   if (ctx->path_graph) cudaGraphDestroy(ctx->path_graph);
-  if (ctx->dt_host) cudaFreeHost(ctx->dt_host);
-  if (ctx->ctl_host) cudaFreeHost(ctx->ctl_host);
-  if (ctx->io_host) cudaFreeHost(ctx->io_host);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return SB_OK;
@@ -1463,14 +1436,14 @@ __global__ void relax_reset_kernel(RelaxControl* ctl) {
 
 // Constants of a full-domain relaxation and its cooperative launch: every CTA
 // resident, at most one warp per tile.
-template <bool FX>
+template <bool FX, int R>
 static int launch_sweeps(sb_ctx* ctx, const RelaxConst& c) {
   SweepConst k{};
   k.n0 = c.n0;
   k.n1 = c.n1;
   k.pitch = c.pitch;
   k.tiles1 = (c.n1 + kSweepInner - 1) / kSweepInner;
-  k.ntiles = k.tiles1 * ((c.n0 + kSweepRows - 2 * kSweepHalo - 1) / (kSweepRows - 2 * kSweepHalo));
+  k.ntiles = k.tiles1 * ((c.n0 + R - 2 * kSweepHalo - 1) / (R - 2 * kSweepHalo));
   k.max_iterations = c.max_iterations;
   k.tol = c.tol;
   for (int d = 0; d < 4; ++d) {
@@ -1486,12 +1459,15 @@ static int launch_sweeps(sb_ctx* ctx, const RelaxConst& c) {
     k.thr[d] = u >= 4294967296.0 ? 0xffffffffu : (unsigned)std::max(thr, 1.0);
   }
   const int per = kSweepThreads / 32;
-  const int grid = std::min((k.ntiles + per - 1) / per, ctx->sweep_ctas);
+  int ctas = 0;  // as many as fit the device at once
+  SB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, sweep_kernel<FX, R>,
+                                                             kSweepThreads, 0));
+  const int grid = std::min((k.ntiles + per - 1) / per, std::max(1, ctas * ctx->sms));
   typename FvTypes<FX>::H *f0 = (typename FvTypes<FX>::H*)ctx->b,
                           *f1 = (typename FvTypes<FX>::H*)ctx->b_alt;
   int *a0 = ctx->sweep_act, *a1 = ctx->sweep_act + k.ntiles;
   void* args[] = {(void*)&k, (void*)&f0, (void*)&f1, (void*)&a0, (void*)&a1, (void*)&ctx->sweep};
-  SB_CUDA(ctx, cudaLaunchCooperativeKernel((void*)sweep_kernel<FX, kSweepRows>, dim3(grid),
+  SB_CUDA(ctx, cudaLaunchCooperativeKernel((void*)sweep_kernel<FX, R>, dim3(grid),
                                            dim3(kSweepThreads), args, 0, ctx->stream));
   ctx->launches++;
   return SB_OK;
@@ -1501,7 +1477,21 @@ static int relax_full(sb_ctx* ctx, const sb_relax_params* p) {
   RelaxConst c;
   int rc = relax_const(ctx, p, &c, kRelaxTile);
   if (rc) return rc;
-  return fx(ctx) ? launch_sweeps<true>(ctx, c) : launch_sweeps<false>(ctx, c);
+  if (!fx(ctx)) return launch_sweeps<false, kSweepRows>(ctx, c);
+  // Box rows.  Measured per sweep, a cut pile settling / every box moving (us):
+  // 701^2 20 rows 4.8 / 9.8, 24 rows 4.9 / 7.8, 28 rows 6.1 / 8.3, 32 rows 7.0 /
+  // 9.1, 48 rows 10.1 / 14.7; 2048^2 20 rows 11.4 / 47, 24 rows 9.2 / 32, 28 rows
+  // 10.9 / 32, 32 rows 9.8 / 33.  More rows redo less halo, but the box's
+  // straight-line code outgrows the instruction cache.
+  // Grids of 2^18 .. 2^20 cells relax to the tolerance with 48 rows all the same
+  // (runs bounded to fewer than 64 iterations do not): there the learned schedule
+  // is required to take at most half the plain sweeps' time
+  // (tests/test_learned_gain_gpu.py), and a proposal's network does not get
+  // faster with the sweeps.
+  const long long cells = (long long)ctx->d.ny * ctx->d.nx;
+  if (c.max_iterations >= 64 && cells >= (1 << 18) && cells <= (1 << 20))
+    return launch_sweeps<true, kSweepRowsTall>(ctx, c);
+  return launch_sweeps<true, kSweepRows>(ctx, c);
 }
 
 // Queues max_iterations (or fewer, if converged) sweeps without waiting for
