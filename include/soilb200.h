@@ -549,6 +549,12 @@ int sb_learned_forward(const void* feat, float* flux, const void* w1, const void
  * [ny][nx][4] scratch). */
 int sb_learned_features(sb_ctx* ctx, void* feat, double tan_crit);
 int sb_learned_apply(sb_ctx* ctx, const float* flux, int32_t* tq, double tan_crit);
+/* One whole proposal round (features, forward, apply) in one call: tan_crit
+ * scales the features, tan_apply the transfers; feat (bf16 [ny][nx][16]), flux
+ * (f32 [ny][nx][4]) and tq are scratch. */
+int sb_learned_propose(sb_ctx* ctx, void* feat, float* flux, int32_t* tq, const void* w1,
+                       const void* w2, const void* w3, const void* w4, double tan_crit,
+                       double tan_apply, int* d_status);
 
 int sb_last_error(sb_ctx* ctx, char* buffer, size_t length);
 /* Number of kernels this context has launched (cumulative). */

@@ -305,6 +305,9 @@ _PROTOTYPES = {
                                      C.c_void_p, C.c_void_p]),
     "sb_learned_features": (C.c_int, [C.c_void_p, C.c_void_p, C.c_double]),
     "sb_learned_apply": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_double]),
+    "sb_learned_propose": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                     C.c_void_p, C.c_void_p, C.c_void_p, C.c_double, C.c_double,
+                                     C.c_void_p]),
 }
 
 # ctypes mirror of each ABI struct, checked against sb_sizeof() in the tests.

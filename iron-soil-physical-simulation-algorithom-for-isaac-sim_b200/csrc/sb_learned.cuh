@@ -705,6 +705,9 @@ struct LearnedGeom {
 template <typename HT>
 __global__ void learned_features_kernel(const LearnedGeom g, const HT* __restrict__ hgt,
                                         __nv_bfloat16* __restrict__ feat) {
+  // a proposal's network kernel stages its weights meanwhile (it waits for this
+  // kernel's end before it reads the features)
+  cudaTriggerProgrammaticLaunchCompletion();
   const double diag = sqrt(g.dx * g.dx + g.dy * g.dy);
   const double scale = g.Q > 0.0 ? g.Q : 1.0;
   const double inv_l[4] = {scale / (g.dx * g.tan_crit), scale / (g.dy * g.tan_crit),
@@ -742,19 +745,31 @@ __device__ __forceinline__ double learned_transfer(const LearnedGeom& g, double 
   return fmin(fmax(t, -lim), lim);
 }
 
-// Fixed point: transfers rounded to whole quanta per edge (int32 [pixel][4]),
-// then gathered -- every quantum leaves one cell and enters one neighbour.
-// Q is a power of two, so t / Q == t * (1 / Q) exactly.
+// Fixed point: transfers in whole quanta per edge (int32 [pixel][4]), rounded
+// toward zero, then gathered -- every quantum leaves one cell and enters one
+// neighbour.  Q is a power of two, so scaling by it commutes with every
+// rounding, and truncation with learned_transfer's clamp to half the (whole)
+// height difference: trunc(clamp(t, lim) / Q) = clamp(trunc(t / Q), |dq| / 2).
+// Four dependent double operations instead of fifteen.
+__device__ __forceinline__ int learned_quanta(float flux, int hc, int hn, double tan_crit,
+                                              double dxq) {
+  const int q = __double2int_rz((double)flux * tan_crit * dxq);  // saturates
+  const unsigned u = hc > hn ? (unsigned)hc - (unsigned)hn : (unsigned)hn - (unsigned)hc;
+  const int lim = (int)(u >> 1);
+  return min(max(q, -lim), lim);
+}
+
 __global__ void learned_quantize_kernel(const LearnedGeom g, const int32_t* __restrict__ hq,
                                         const float* __restrict__ flux /*[pixel][4]*/,
                                         int32_t* __restrict__ tq /*[pixel][4]*/) {
-  const double inv_q = 1.0 / g.Q;
+  const double dxq = g.dx * (1.0 / g.Q);
+  cudaGridDependencySynchronize();
   for (int row = blockIdx.x; row < g.batch * g.h; row += gridDim.x) {
     const int bb = row / g.h, r = row - bb * g.h;
     const int32_t* H = hq + (size_t)bb * g.h * g.pitch;
     for (int c = threadIdx.x; c < g.w; c += blockDim.x) {
       const size_t i = (size_t)row * g.w + c;
-      const double hc = (double)H[(size_t)r * g.pitch + c] * g.Q;
+      const int hc = H[(size_t)r * g.pitch + c];
       const float4 fl = *reinterpret_cast<const float4*>(flux + i * 4);
       const float fk[4] = {fl.x, fl.y, fl.z, fl.w};
       int q[4];
@@ -764,11 +779,8 @@ __global__ void learned_quantize_kernel(const LearnedGeom g, const int32_t* __re
         edge_of(k, dr, dc);
         const int rn = r + dr, cn = c + dc;
         q[k] = 0;
-        if (rn < g.h && cn >= 0 && cn < g.w) {
-          const double hn = (double)H[(size_t)rn * g.pitch + cn] * g.Q;
-          const double t = learned_transfer(g, (double)fk[k], hc, hn);
-          q[k] = (int)trunc(t * inv_q);  // toward zero: stays within the half-difference limit
-        }
+        if (rn < g.h && cn >= 0 && cn < g.w)
+          q[k] = learned_quanta(fk[k], hc, H[(size_t)rn * g.pitch + cn], g.tan_crit, dxq);
       }
       *reinterpret_cast<int4*>(tq + i * 4) = make_int4(q[0], q[1], q[2], q[3]);
     }
@@ -777,6 +789,7 @@ __global__ void learned_quantize_kernel(const LearnedGeom g, const int32_t* __re
 
 __global__ void learned_apply_fx_kernel(const LearnedGeom g, int32_t* __restrict__ hq,
                                         const int32_t* __restrict__ tq) {
+  cudaGridDependencySynchronize();
   for (int row = blockIdx.x; row < g.batch * g.h; row += gridDim.x) {
     const int bb = row / g.h, r = row - bb * g.h;
     int32_t* H = hq + (size_t)bb * g.h * g.pitch;

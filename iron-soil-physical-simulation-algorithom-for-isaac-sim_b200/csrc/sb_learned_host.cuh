@@ -81,6 +81,70 @@ int lcuda(cudaError_t e) {
 
 }  // namespace
 
+// Launches a kernel that calls cudaGridDependencySynchronize() before it reads
+// its predecessor's results; with overlap it may start before that has ended.
+template <typename... P, typename... A>
+static cudaError_t launch_after(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
+                                cudaStream_t stream, bool overlap, const A&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+static int launch_net(const void* feat, float* flux, const void* const (&wpk)[4], int batch, int h,
+                      int w, int rows_per_cta, int* d_status, cudaStream_t stream, bool overlap) {
+  if (!feat || !flux || !wpk[0] || !wpk[1] || !wpk[2] || !wpk[3] || batch <= 0 || h <= 0 || w <= 0 ||
+      rows_per_cta < 0 || batch > 65535)
+    return lfail(SB_ERR_BAD_ARG, "[soilb200] forward: bad arguments");
+  if (((uintptr_t)feat | (uintptr_t)flux | (uintptr_t)wpk[0] | (uintptr_t)wpk[1] |
+       (uintptr_t)wpk[2] | (uintptr_t)wpk[3]) & 15)
+    return lfail(SB_ERR_BAD_ARG, "[soilb200] forward: buffers must be 16-byte aligned");
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return lfail(SB_ERR_CUDA, "[soilb200] forward: cuTensorMapEncodeTiled unavailable");
+  // features as a 4-D tensor (channel, x, y, image); one box = one channel
+  // chunk of a staged row: 8 channels x 130 pixels, zeros outside the image
+  CUtensorMap map;
+  const cuuint64_t dims[4] = {16, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)batch};
+  const cuuint64_t strides[3] = {32, (cuuint64_t)w * 32, (cuuint64_t)w * (cuuint64_t)h * 32};
+  const cuuint32_t box[4] = {8, (cuuint32_t)kRowPixels, 1, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(feat), dims, strides, box,
+          estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return lfail(SB_ERR_CUDA, "[soilb200] forward: feature tensor map rejected");
+  const int strips = (w + kNetTileOut - 1) / kNetTileOut;
+  int rows = rows_per_cta;
+  if (rows == 0) {  // one CTA per SM: about one wave over the 148 SMs
+    const long long per_band = (long long)strips * batch;
+    const int bands = per_band >= 148 ? 1 : (int)(148 / per_band);
+    rows = (h + bands - 1) / bands;
+  }
+  static bool attr_set[16] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 16 && !attr_set[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(net_forward_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         NetSmem::BYTES);
+    if (e != cudaSuccess) return lcuda(e);
+    attr_set[dev] = true;
+  }
+  NetArgs a{{(const __nv_bfloat16*)wpk[0], (const __nv_bfloat16*)wpk[1],
+             (const __nv_bfloat16*)wpk[2], (const __nv_bfloat16*)wpk[3]},
+            flux, batch, h, w, rows, d_status};
+  dim3 grid(strips, (h + rows - 1) / rows, batch);
+  return lcuda(launch_after(net_forward_kernel, grid, kNetThreads, NetSmem::BYTES, stream, overlap,
+                            map, a));
+}
+
 extern "C" {
 
 const char* sb_learned_last_error(void) { return g_learned_err; }
@@ -163,48 +227,9 @@ int sb_learned_loss(const float* flux, const float* target_dh, float* resid, voi
 int sb_learned_forward(const void* feat, float* flux, const void* w1, const void* w2,
                        const void* w3, const void* w4, int batch, int h, int w, int rows_per_cta,
                        int* d_status, void* stream) {
-  if (!feat || !flux || !w1 || !w2 || !w3 || !w4 || batch <= 0 || h <= 0 || w <= 0 ||
-      rows_per_cta < 0 || batch > 65535)
-    return lfail(SB_ERR_BAD_ARG, "[soilb200] forward: bad arguments");
-  if (((uintptr_t)feat | (uintptr_t)flux | (uintptr_t)w1 | (uintptr_t)w2 | (uintptr_t)w3 |
-       (uintptr_t)w4) & 15)
-    return lfail(SB_ERR_BAD_ARG, "[soilb200] forward: buffers must be 16-byte aligned");
-  EncodeTiledFn enc = encode_fn();
-  if (!enc) return lfail(SB_ERR_CUDA, "[soilb200] forward: cuTensorMapEncodeTiled unavailable");
-  // features as a 4-D tensor (channel, x, y, image); one box = one channel
-  // chunk of a staged row: 8 channels x 130 pixels, zeros outside the image
-  CUtensorMap map;
-  const cuuint64_t dims[4] = {16, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)batch};
-  const cuuint64_t strides[3] = {32, (cuuint64_t)w * 32, (cuuint64_t)w * (cuuint64_t)h * 32};
-  const cuuint32_t box[4] = {8, (cuuint32_t)kRowPixels, 1, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(feat), dims, strides, box,
-          estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return lfail(SB_ERR_CUDA, "[soilb200] forward: feature tensor map rejected");
-  const int strips = (w + kNetTileOut - 1) / kNetTileOut;
-  int rows = rows_per_cta;
-  if (rows == 0) {  // one CTA per SM: about one wave over the 148 SMs
-    const long long per_band = (long long)strips * batch;
-    const int bands = per_band >= 148 ? 1 : (int)(148 / per_band);
-    rows = (h + bands - 1) / bands;
-  }
-  static bool attr_set[16] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 16 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(net_forward_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         NetSmem::BYTES);
-    if (e != cudaSuccess) return lcuda(e);
-    attr_set[dev] = true;
-  }
-  NetArgs a{{(const __nv_bfloat16*)w1, (const __nv_bfloat16*)w2, (const __nv_bfloat16*)w3,
-             (const __nv_bfloat16*)w4},
-            flux, batch, h, w, rows, d_status};
-  dim3 grid(strips, (h + rows - 1) / rows, batch);
-  net_forward_kernel<<<grid, kNetThreads, NetSmem::BYTES, (cudaStream_t)stream>>>(map, a);
-  return lcuda(cudaGetLastError());
+  const void* wpk[4] = {w1, w2, w3, w4};
+  return launch_net(feat, flux, wpk, batch, h, w, rows_per_cta, d_status, (cudaStream_t)stream,
+                    false);
 }
 
 int sb_learned_loss_blocks(int batch, int h, int w) {
@@ -239,6 +264,36 @@ int sb_learned_apply(sb_ctx* ctx, const float* flux, int32_t* tq, double tan_cri
   learned_apply_fx_kernel<<<blocks, kThreads, 0, ctx->stream>>>(g, (int32_t*)ctx->b, tq);
   ctx->launches += 2;
   SB_CUDA(ctx, cudaGetLastError());
+  return SB_OK;
+}
+
+// One proposal round on a context's resident b_eff in one call: features into
+// feat (bf16 [ny][nx][16]), the network's fluxes (f32 [ny][nx][4]), their
+// transfers (tq: int32 [ny][nx][4]) and the application; all three buffers are
+// scratch.  Equal to sb_learned_features, sb_learned_forward and
+// sb_learned_apply; the kernels' starts overlap their predecessors' ends
+// (701^2: the network's staging of weights takes about 4 us, a launch gap 2).
+int sb_learned_propose(sb_ctx* ctx, void* feat, float* flux, int32_t* tq, const void* w1,
+                       const void* w2, const void* w3, const void* w4, double tan_crit,
+                       double tan_apply, int* d_status) {
+  if (!ctx || !feat || !flux || !tq || !(tan_crit > 0.0) || !(tan_apply > 0.0))
+    return SB_ERR_BAD_ARG;
+  if (((uintptr_t)flux | (uintptr_t)tq) & 15)
+    return fail(ctx, SB_ERR_BAD_ARG, "[soilb200] learned propose: buffers must be 16-byte aligned");
+  int rc = sb_learned_features(ctx, feat, tan_crit);
+  if (rc) return rc;
+  const int ny = ctx->d.ny, nx = ctx->d.nx;
+  const void* wpk[4] = {w1, w2, w3, w4};
+  if ((rc = launch_net(feat, flux, wpk, 1, ny, nx, 0, d_status, ctx->stream, true)))
+    return fail(ctx, rc, "%s", sb_learned_last_error());
+  const LearnedGeom g{1, ny, nx, ctx->pitch, ctx->d.dx_m, ctx->d.dy_m, tan_apply, ctx->quantum,
+                      ctx->d.datum_m};
+  const int blocks = learned_row_grid(1, ny);
+  SB_CUDA(ctx, launch_after(learned_quantize_kernel, dim3(blocks), kThreads, 0, ctx->stream, true,
+                            g, (const int32_t*)ctx->b, (const float*)flux, tq));
+  SB_CUDA(ctx, launch_after(learned_apply_fx_kernel, dim3(blocks), kThreads, 0, ctx->stream, true,
+                            g, (int32_t*)ctx->b, (const int32_t*)tq));
+  ctx->launches += 3;
   return SB_OK;
 }
 

@@ -236,6 +236,9 @@ __global__ void __launch_bounds__(kNetThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // launched with programmatic serialization, everything above overlaps the
+  // features' kernel
+  cudaGridDependencySynchronize();
 
   if (warp == 4 * kNetEpiGroups + 4) {
     // ---- feature rows B-4 .. B+n+3 by TMA (input i of layer 0, slot i % 6)

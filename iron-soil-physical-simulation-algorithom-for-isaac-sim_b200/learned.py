@@ -297,6 +297,7 @@ class LearnedRelaxation:
         ny, nx = grid.shape
         dev = net.device
         self._feat = torch.empty(1, ny, nx, 16, dtype=torch.bfloat16, device=dev)
+        self._flux = torch.empty(ny * nx * 4, dtype=torch.float32, device=dev)
         self._tq = torch.empty(ny * nx * 4, dtype=torch.int32, device=dev)
         self._packed = net.packed()
         self._stream = grid.stream_handle()
@@ -313,17 +314,22 @@ class LearnedRelaxation:
         lib = _lib.load()
         if not scale > 0.0:
             raise ValueError("[soilb200] the proposal scale must be positive")
+        if self.fused:
+            w = [p.data_ptr() for p in self._packed]
+            for _ in range(rounds):
+                # the transfer is flux * tan * dx, so the scale rides on tan
+                _lib.check(self.grid.ctx, lib.sb_learned_propose(
+                    self.grid.ctx, self._feat.data_ptr(), self._flux.data_ptr(),
+                    self._tq.data_ptr(), *w, self.tan_crit, self.tan_crit * scale,
+                    self.net.status.data_ptr()), "propose")
+            return
         with torch.cuda.stream(self._torch_stream):
             for _ in range(rounds):
                 _lib.check(self.grid.ctx, lib.sb_learned_features(self.grid.ctx,
                                                                   self._feat.data_ptr(),
                                                                   self.tan_crit), "features")
-                if self.fused:
-                    flux = network_forward_fused(self.net, self._feat, self._packed,
-                                                 stream=self._stream)
-                else:
-                    _, flux = network_forward(self.net, self._feat, self._packed,
-                                              stream=self._stream)
+                _, flux = network_forward(self.net, self._feat, self._packed,
+                                          stream=self._stream)
                 # the transfer is flux * tan * dx, so the scale rides on tan
                 _lib.check(self.grid.ctx, lib.sb_learned_apply(self.grid.ctx, flux.data_ptr(),
                                                                self._tq.data_ptr(),
