@@ -11,7 +11,7 @@
 #include "sb_exchange.cuh"
 #include "sb_labels.cuh"
 #include "sb_ledger.cuh"
-#include "sb_relax.cuh"
+#include "sb_frontier.cuh"
 
 namespace sb {
 
@@ -288,8 +288,6 @@ __device__ __forceinline__ void path_classify_body(const PathConst& c, const Lab
   rctl->n_active = 0;
   rctl->rounds = 0;
   rctl->moved_edges = 0;
-  rctl->list_len = 0;
-  rctl->sub_len = 0;
 }
 
 // The component reduction and, in the thread that finishes it, the
@@ -305,16 +303,12 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Previous-candidate mask and frontier seeds of the winner; the last block
-// to finish then opens the residual frontier loop (frontier_begin).
+// Previous-candidate mask and frontier seeds of the winner.
 __global__ void __launch_bounds__(kThreads)
     path_update_previous_kernel(const LabelConst c, const int* __restrict__ parent,
                                 int* __restrict__ previous, int* __restrict__ reached,
                                 int* __restrict__ tile_flags, const LabelOut* out,
-                                const PathState* ps, const RelaxConst rc, int* __restrict__ phase0,
-                                int* __restrict__ phase1, RelaxControl* rctl,
-                                cudaGraphConditionalHandle handle) {
-  __shared__ int last;
+                                const PathState* ps) {
   const int n = c.ny * c.nx;
   const int winner = out->winner;
   const int keep = ps->keep_candidate, seed = ps->seed_frontier;
@@ -327,41 +321,6 @@ __global__ void __launch_bounds__(kThreads)
       tile_flags[(r / c.tile_size) * c.frontier_tiles_x + col / c.tile_size] = 1;
     }
   }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(&rctl->arrive, 1u) == gridDim.x - 1) ? 1 : 0;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (threadIdx.x == 0) rctl->arrive = 0;
-  frontier_begin_body(rc, tile_flags, phase0, phase1, rctl, handle);
-}
-
-// Step end: the step's records into the caller-visible pinned host copies
-// (device-mapped pointers, one launch instead of one copy per record), and the
-// reached mask cleared after a converged residual (frontier_finish).
-struct PathRecordPtrs {
-  const void* src[6];
-  void* dst[6];
-  int bytes[6];
-};
-
-__global__ void __launch_bounds__(kThreads)
-    path_records_kernel(const PathRecordPtrs p, const RelaxConst rc, int* __restrict__ reached,
-                        const RelaxControl* rctl) {
-  if (blockIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) {
-      const unsigned* s = static_cast<const unsigned*>(p.src[k]);
-      unsigned* d = static_cast<unsigned*>(p.dst[k]);
-      for (int w = threadIdx.x; w < p.bytes[k] / 4; w += blockDim.x) d[w] = __ldcg(s + w);
-    }
-    __threadfence_system();
-  }
-  if (!rctl->converged) return;
-  const long long n = (long long)rc.n0 * rc.pitch;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    reached[i] = 0;
 }
 
 // The standalone Mobile V2 step graph's ends: dt from the host-mapped input
@@ -374,13 +333,6 @@ __global__ void fv_begin_mapped_kernel(FvControl* ctl, const double* dt_mapped, 
   }
 }
 
-__global__ void records_copy_kernel(const PathRecordPtrs p, int n) {
-  for (int k = 0; k < n; ++k) {
-    const unsigned* s = static_cast<const unsigned*>(p.src[k]);
-    unsigned* d = static_cast<unsigned*>(p.dst[k]);
-    for (int w = threadIdx.x; w < p.bytes[k] / 4; w += blockDim.x) d[w] = __ldcg(s + w);
-  }
-  __threadfence_system();
-}
+__global__ void records_copy_kernel(const PathRecordPtrs p, int n) { copy_records(p, n); }
 
 }  // namespace sb

@@ -190,10 +190,12 @@ struct sb_ctx {
   int* reached_alt = nullptr;
   int ftiles0 = 0, ftiles1 = 0;
   int* ftile_next = nullptr;   // next-round active tiles (seeded by labels / seeds)
-  // residual frontier: phase[0] = the round's tile membership flags,
-  // phase[1] = the round's compacted tile list (both ntiles ints)
-  int* phase[2] = {nullptr, nullptr};
-  int frontier_grid = 1;  // CTAs of the list-driven frontier kernels
+  // residual frontier: tile stamps and the two rounds' tile lists (ntiles ints
+  // each), barrier words, CTAs of the launch
+  int* ftile_stamp = nullptr;
+  int* ftile_list[2] = {nullptr, nullptr};
+  FrontierSync* fsync = nullptr;
+  int frontier_grid = 1;
   RelaxControl* rctl = nullptr;
   RelaxControl* rctl_host = nullptr;
   // full-domain sweeps: loop control, per-tile change flags (two iterations)
@@ -202,7 +204,6 @@ struct sb_ctx {
   int* sweep_act = nullptr;
   int sms = 1;
   LoopGraph relax_reached;  // reached-gated (event-driven) sweep to tolerance
-  LoopGraph frontier;
   // fused plain-path step
   PathState* pstate = nullptr;
   PathState* pstate_host = nullptr;
@@ -845,19 +846,25 @@ int sb_ctx_create(const sb_grid_desc* desc, sb_ctx** out) {
   ctx->ftiles0 = (d.ny + d.tile_size - 1) / d.tile_size;
   ctx->ftiles1 = (d.nx + d.tile_size - 1) / d.tile_size;
   {
-    // list-driven frontier kernels: eight 256-thread CTAs per SM stride over
-    // the active tiles (never more CTAs than tiles)
-    int sms = 0;
+    // one pair of a sub-phase per thread with every tile active, at most two
+    // CTAs per SM (a barrier's time grows with its CTAs)
+    int sms = 0, per_sm = 0;
     SB_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d.device));
-    ctx->frontier_grid =
-        (int)std::min<long long>((long long)ctx->ftiles0 * ctx->ftiles1, 8LL * std::max(sms, 1));
+    const void* fn = fx(ctx) ? (const void*)frontier_kernel<true> : (const void*)frontier_kernel<false>;
+    SB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, 0));
+    const long long pairs =
+        (long long)ctx->ftiles0 * ctx->ftiles1 * ((d.tile_size + 1) / 2) * d.tile_size;
+    ctx->frontier_grid = (int)std::max(1LL, std::min({(pairs + kThreads - 1) / kThreads,
+                                                      2LL * sms, (long long)per_sm * sms}));
   }
   const size_t nt = (size_t)ctx->ftiles0 * ctx->ftiles1;
   dev.add(&ctx->ptiles, nt * sizeof(int));
   dev.add(&ctx->dtiles, nt * sizeof(int));
   dev.add(&ctx->ftile_next, nt * 4);
-  dev.add(&ctx->phase[0], nt * 4);
-  dev.add(&ctx->phase[1], nt * 4);
+  dev.add(&ctx->ftile_stamp, nt * 4);
+  dev.add(&ctx->ftile_list[0], nt * 4);
+  dev.add(&ctx->ftile_list[1], nt * 4);
+  dev.add(&ctx->fsync, sizeof(FrontierSync));
   {
     SB_CUDA(ctx, cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, d.device));
     const int inner = kSweepRows - 2 * kSweepHalo;
@@ -951,7 +958,6 @@ int sb_ctx_destroy(sb_ctx* ctx) {
   if (ctx->mobile.exec) cudaGraphExecDestroy(ctx->mobile.exec);
   if (ctx->mobile.graph) cudaGraphDestroy(ctx->mobile.graph);
   ctx->relax_reached.reset();
-  ctx->frontier.reset();
   void* ptrs[] = {ctx->arena, ctx->q_rows, ctx->q_cols, ctx->q_out};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1429,8 +1435,6 @@ __global__ void relax_reset_kernel(RelaxControl* ctl) {
     ctl->n_active = 0;
     ctl->rounds = 0;
     ctl->moved_edges = 0;
-    ctl->list_len = 0;
-    ctl->sub_len = 0;
   }
 }
 
@@ -1710,99 +1714,50 @@ extern "C" int sb_frontier_active_tiles(sb_ctx* ctx, int32_t* flags, int capacit
   return SB_OK;
 }
 
-template <bool FX>
-static int build_frontier(sb_ctx* ctx, const RelaxConst& c) {
-  LoopGraph& lg = ctx->frontier;
-  lg.reset();
-  cudaGraph_t g;
-  SB_CUDA(ctx, cudaGraphCreate(&g, 0));
-  lg.graph = g;
-  cudaGraphConditionalHandle handle;
-  SB_CUDA(ctx, cudaGraphConditionalHandleCreate(&handle, g, 0, cudaGraphCondAssignDefault));
-  RelaxConst cc;  // copied into the node parameters at add time
-  cc = c;
-  cudaGraphNode_t n_reset, n_begin0, n_loop, n_finish;
-  int rc;
-  {
-    void* args[] = {(void*)&ctx->rctl};
-    if ((rc = add_kernel(ctx, g, &n_reset, nullptr, 0, (void*)relax_reset_kernel, dim3(1), 0, args)))
-      return rc;
+// Arguments of the frontier kernel; the referenced locals must outlive the launch.
+struct FrontierArgs {
+  RelaxConst c;
+  PathRecordPtrs rec{};
+  int nrec = 0;
+  std::vector<void*> list;
+  FrontierArgs(sb_ctx* ctx, const RelaxConst& rc) : c(rc) {
+    list = {&c,
+            &ctx->b,
+            &ctx->reached,
+            &ctx->ftile_next,
+            &ctx->ftile_stamp,
+            &ctx->ftile_list[0],
+            &ctx->ftile_list[1],
+            &ctx->rctl,
+            &ctx->fsync,
+            &rec,
+            &nrec};
   }
-  void* begin_args[] = {(void*)&cc, (void*)&ctx->ftile_next, (void*)&ctx->phase[0],
-                        (void*)&ctx->phase[1], (void*)&ctx->rctl, (void*)&handle};
-  if ((rc = add_kernel(ctx, g, &n_begin0, &n_reset, 1, (void*)frontier_begin_kernel, dim3(1), 0,
-                       begin_args)))
-    return rc;
-  cudaGraphNodeParams cp{};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = handle;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  SB_CUDA(ctx, cudaGraphAddNode(&n_loop, g, &n_begin0, 1, &cp));
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  cudaGraphNode_t prev = nullptr;
-  int dirs[8], pars[8];
-  for (int k = 0; k < 8; ++k) {
-    dirs[k] = k / 2;
-    pars[k] = k % 2;
-  }
-  typename FvTypes<FX>::H* hf = (typename FvTypes<FX>::H*)ctx->b;
-  for (int k = 0; k < 8; ++k) {
-    cudaGraphNode_t node;
-    void* args[] = {(void*)&cc, (void*)&dirs[k], (void*)&pars[k], (void*)&hf,
-                    (void*)&ctx->reached, (void*)&ctx->phase[0], (void*)&ctx->phase[1],
-                    (void*)&ctx->rctl};
-    if ((rc = add_kernel(ctx, body, &node, prev ? &prev : nullptr, prev ? 1 : 0,
-                         (void*)frontier_subphase_kernel<FX>, dim3(ctx->frontier_grid), 0,
-                         args)))
-      return rc;
-    prev = node;
-  }
-  cudaGraphNode_t n_scan, n_begin;
-  {
-    void* args[] = {(void*)&cc, (void*)&hf, (void*)&ctx->reached, (void*)&ctx->phase[1],
-                    (void*)&ctx->ftile_next, (void*)&ctx->rctl};
-    if ((rc = add_kernel(ctx, body, &n_scan, &prev, 1, (void*)frontier_scan_kernel<FX>,
-                         dim3(ctx->frontier_grid), 0, args)))
-      return rc;
-  }
-  if ((rc = add_kernel(ctx, body, &n_begin, &n_scan, 1, (void*)frontier_begin_kernel, dim3(1), 0,
-                       begin_args)))
-    return rc;
-  {
-    void* args[] = {(void*)&cc, (void*)&ctx->reached, (void*)&ctx->rctl};
-    if ((rc = add_kernel(ctx, g, &n_finish, &n_loop, 1, (void*)frontier_finish_kernel,
-                         dim3(grid_for((long long)c.n0 * c.pitch)), 0, args)))
-      return rc;
-  }
-  SB_CUDA(ctx, cudaGraphInstantiate(&lg.exec, g, 0));
-  lg.key = c;
-  lg.valid = true;
-  return SB_OK;
-}
+};
 
 extern "C" int sb_frontier_run(sb_ctx* ctx, const sb_relax_params* p, sb_relax_stats* out) {
   if (!ctx || !p || !out) return SB_ERR_BAD_ARG;
   RelaxConst c;
   int rc = relax_const(ctx, p, &c, ctx->d.tile_size);
   if (rc) return rc;
-  LoopGraph& lg = ctx->frontier;
-  if (!lg.valid || std::memcmp(&lg.key, &c, sizeof(RelaxConst)) != 0) {
-    rc = fx(ctx) ? build_frontier<true>(ctx, c) : build_frontier<false>(ctx, c);
-    if (rc) return rc;
-  }
-  SB_CUDA(ctx, cudaGraphLaunch(lg.exec, ctx->stream));
+  FrontierArgs args(ctx, c);
+  relax_reset_kernel<<<1, kThreads, 0, ctx->stream>>>(ctx->rctl);
+  SB_CUDA(ctx, cudaLaunchCooperativeKernel(
+                   fx(ctx) ? (void*)frontier_kernel<true> : (void*)frontier_kernel<false>,
+                   dim3(ctx->frontier_grid), dim3(kThreads), args.list.data(), 0, ctx->stream));
   SB_CUDA(ctx, cudaMemcpyAsync(ctx->rctl_host, ctx->rctl, sizeof(RelaxControl),
                                cudaMemcpyDeviceToHost, ctx->stream));
   SB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   const RelaxControl& k = *ctx->rctl_host;
-  ctx->launches += 3 + 10LL * k.rounds;
+  ctx->launches += 2;
   std::memset(out, 0, sizeof(*out));
   out->iterations = k.rounds;
   out->converged = k.converged;
   out->status = k.status;
   out->active_tiles = k.n_active;
   out->moved_edges = k.moved_edges;
+  if (k.status == SB_ERR_WAIT_LIMIT)
+    return fail(ctx, SB_ERR_WAIT_LIMIT, "[soilb200] a bounded device wait gave up (frontier barrier)");
   if (k.status == SB_ERR_NONCONVERGENCE)
     return fail(ctx, SB_ERR_NONCONVERGENCE,
                 "NUMERICAL_NONCONVERGENCE: GPU residual MiniSlope exceeded the numerical safety limit");
@@ -2210,13 +2165,12 @@ int build_path_graph(sb_ctx* ctx, const sb_path_params* p) {
   cudaGraph_t g;
   SB_CUDA(ctx, cudaGraphCreate(&g, 0));
   ctx->path_graph = g;
-  cudaGraphConditionalHandle h_mob, h_front;
+  cudaGraphConditionalHandle h_mob;
   // a conditional handle without a conditional node can fail instantiation:
   // the persistent substep loop needs none
   h_mob = 0;
   if (!(FX && ctx->fv_stream && ctx->fv_persistent))
     SB_CUDA(ctx, cudaGraphConditionalHandleCreate(&h_mob, g, 0, cudaGraphCondAssignDefault));
-  SB_CUDA(ctx, cudaGraphConditionalHandleCreate(&h_front, g, 0, cudaGraphCondAssignDefault));
   int rc, one = 1, zero = 0;
   const int ny = ctx->d.ny, nx = ctx->d.nx;
   double Q = ctx->quantum, datum = ctx->d.datum_m, f = ctx->d.dx_m * ctx->d.dy_m / 6.0;
@@ -2374,56 +2328,21 @@ int build_path_graph(sb_ctx* ctx, const sb_path_params* p) {
     prev = node;
     if ((rc = mark())) return rc;
   }
-  // 5. previous mask + frontier seeds; its last block opens the gated
-  // residual frontier loop (same kernels as sb_frontier_run)
-  void* begin_args[] = {&rcn, &ctx->ftile_next, &ctx->phase[0], &ctx->phase[1], &ctx->rctl,
-                        &h_front};
+  // 5. previous mask + frontier seeds
   {
     void* args[] = {&lc, &ctx->parent, &ctx->previous, &ctx->reached, &ctx->ftile_next, &ctx->lout,
-                    &ctx->pstate, &rcn, &ctx->phase[0], &ctx->phase[1], &ctx->rctl, &h_front};
+                    &ctx->pstate};
     if ((rc = add_kernel(ctx, g, &node, &prev, 1, (void*)path_update_previous_kernel,
                          dim3(grid_for((long long)ny * nx)), 0, args)))
       return rc;
     prev = node;
     if ((rc = mark())) return rc;
   }
+  // 6. the residual frontier, closed or open by the classification's gate; its
+  // last CTA writes the step's records to the pinned host copies
   {
-    cudaGraphNodeParams cp{};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h_front;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    SB_CUDA(ctx, cudaGraphAddNode(&node, g, &prev, 1, &cp));
-    prev = node;
-    if ((rc = mark())) return rc;
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    int dirs[8], pars[8];
-    typename T::H* hf;
-    hf = (typename T::H*)ctx->b;
-    cudaGraphNode_t bprev = nullptr, bnode;
-    for (int k = 0; k < 8; ++k) {
-      dirs[k] = k / 2;
-      pars[k] = k % 2;
-      void* args[] = {&rcn, &dirs[k], &pars[k], &hf, &ctx->reached, &ctx->phase[0],
-                      &ctx->phase[1], &ctx->rctl};
-      if ((rc = add_kernel(ctx, body, &bnode, bprev ? &bprev : nullptr, bprev ? 1 : 0,
-                           (void*)frontier_subphase_kernel<FX>, dim3(ctx->frontier_grid), 0,
-                           args)))
-        return rc;
-      bprev = bnode;
-    }
-    void* sargs[] = {&rcn, &hf, &ctx->reached, &ctx->phase[1], &ctx->ftile_next, &ctx->rctl};
-    if ((rc = add_kernel(ctx, body, &bnode, &bprev, 1, (void*)frontier_scan_kernel<FX>,
-                         dim3(ctx->frontier_grid), 0, sargs)))
-      return rc;
-    bprev = bnode;
-    if ((rc = add_kernel(ctx, body, &bnode, &bprev, 1, (void*)frontier_begin_kernel, dim3(1), 0,
-                         begin_args)))
-      return rc;
-  }
-  // 6. records to the pinned host copies (+ frontier_finish)
-  {
-    PathRecordPtrs rp;
+    FrontierArgs fa(ctx, rcn);
+    fa.nrec = 6;
     const void* srcs[6] = {ctx->ctl, ctx->io, ctx->lout, ctx->rctl, ctx->pstate, ctx->xout};
     void* hosts[6] = {ctx->ctl_host, ctx->io_host, ctx->lout_host, ctx->rctl_host,
                       ctx->pstate_host, ctx->xout_host};
@@ -2437,15 +2356,18 @@ int build_path_graph(sb_ctx* ctx, const sb_path_params* p) {
                     "records are copied as 32-bit words");
       void* dptr = nullptr;
       SB_CUDA(ctx, cudaHostGetDevicePointer(&dptr, hosts[k], 0));
-      rp.src[k] = srcs[k];
-      rp.dst[k] = dptr;
-      rp.bytes[k] = sizes[k];
+      fa.rec.src[k] = srcs[k];
+      fa.rec.dst[k] = dptr;
+      fa.rec.bytes[k] = sizes[k];
     }
-    void* args[] = {&rp, &rcn, &ctx->reached, &ctx->rctl};
-    if ((rc = add_kernel(ctx, g, &node, &prev, 1, (void*)path_records_kernel,
-                         dim3(std::min(grid_for((long long)rcn.n0 * rcn.pitch), 2 * 148)), 0, args)))
+    if ((rc = add_kernel(ctx, g, &node, &prev, 1, (void*)frontier_kernel<FX>,
+                         dim3(ctx->frontier_grid), 0, fa.list.data())))
       return rc;
+    cudaLaunchAttributeValue coop{};
+    coop.cooperative = 1;
+    SB_CUDA(ctx, cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributeCooperative, &coop));
     prev = node;
+    if ((rc = mark())) return rc;
   }
   SB_CUDA(ctx, cudaGraphAddEventRecordNode(&node, g, &prev, 1, ctx->ev_path[1]));
   (void)one;
@@ -2568,12 +2490,10 @@ extern "C" int sb_path_step(sb_ctx* ctx, double dt_s, const int32_t* cut_idx,
     }
   }
   const FvControl& k = *ctx->ctl_host;
-  // ten kernels outside the loops, two substep launches per loop iteration,
-  // ten kernels per residual round
-  ctx->launches += 10 +
-                   ((fx(ctx) && ctx->fv_stream && ctx->fv_persistent) ? 1
-                                                                      : (k.substeps + 1) / 2 * 2) +
-                   10LL * r.rounds;
+  // nine kernels outside the substep loop, two substep launches per loop iteration
+  ctx->launches += 9 + ((fx(ctx) && ctx->fv_stream && ctx->fv_persistent)
+                            ? 1
+                            : (k.substeps + 1) / 2 * 2);
   if (ctx->xout_host->bad_index)
     return fail(ctx, SB_ERR_BAD_ARG, "[DeviceBulkState] entrainment index outside state");
   if (k.status == SB_ERR_POSITIVITY) return fail(ctx, SB_ERR_POSITIVITY, "MobileV2 positivity failure");
@@ -2582,6 +2502,8 @@ extern "C" int sb_path_step(sb_ctx* ctx, double dt_s, const int32_t* cut_idx,
   if (k.status) return fail(ctx, k.status, "[soilb200] device status %d", k.status);
   if (o.status)
     return fail(ctx, SB_ERR_NONCONVERGENCE, "NUMERICAL_NONCONVERGENCE: device avalanche connected components");
+  if (r.status == SB_ERR_WAIT_LIMIT)
+    return fail(ctx, SB_ERR_WAIT_LIMIT, "[soilb200] a bounded device wait gave up (frontier barrier)");
   if (r.status == SB_ERR_NONCONVERGENCE)
     return fail(ctx, SB_ERR_NONCONVERGENCE,
                 "NUMERICAL_NONCONVERGENCE: GPU residual MiniSlope exceeded the numerical safety limit");
