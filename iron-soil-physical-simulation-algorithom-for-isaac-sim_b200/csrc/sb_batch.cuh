@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kThreads)
   const int n = (r1 - r0) * c.nx;
   for (int i = threadIdx.x; i < n; i += kThreads)
     ledger_cell<true>(c, a.b + base, a.z + base, a.h[parity] + base, a.qx[parity] + base,
-                      a.qy[parity] + base, nullptr, nullptr, P.datum, r0 + i / c.nx, i % c.nx, v,
+                      a.qy[parity] + base, nullptr, nullptr, P.datum, r0 + i / c.nx, i % c.nx, nullptr, v,
                       iq0, iq1, iq2);
   ledger_block_store(v, iq0, iq1, iq2, fold, partials + (size_t)band * L_NP,
                      ipartials + (size_t)band * kLedgerI64, 1);

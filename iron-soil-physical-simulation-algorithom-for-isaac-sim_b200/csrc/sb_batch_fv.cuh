@@ -56,16 +56,14 @@ __global__ void __launch_bounds__(kThreads, 3)
   const int parity = ctl[p].k.parity;
   const int local = gw - P.first_item;
   double acc[kFvDiag];
-#pragma unroll
-  for (int k = 0; k < kFvDiag; ++k) acc[k] = 0.0;
-  double wave = 0.0;
+  float fa[kFvDiag] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, fwave = 0.f;
   fx_strip_run<FAST>(c, a.b + base, a.h[parity] + base, a.qx[parity] + base, a.qy[parity] + base,
                a.h[parity ^ 1] + base, a.qx[parity ^ 1] + base, a.qy[parity ^ 1] + base, nullptr,
                nullptr, local % c.tiles_x, (local / c.tiles_x) * c.rows_per_warp,
-               min((local / c.tiles_x + 1) * c.rows_per_warp, c.ny), sub_dt, acc, wave);
+               min((local / c.tiles_x + 1) * c.rows_per_warp, c.ny), sub_dt, fa, fwave);
 #pragma unroll
-  for (int k = 0; k < kFvDiag; ++k) acc[k] = warp_sum(acc[k]);
-  wave = warp_max(wave);
+  for (int k = 0; k < kFvDiag; ++k) acc[k] = warp_sum((double)fa[k]);
+  const double wave = warp_max((double)fwave);
   if ((threadIdx.x & 31) == 0) {
     double* out = item_partials + (size_t)gw * (kFvDiag + 1);
     for (int k = 0; k < kFvDiag; ++k) out[k] = acc[k];

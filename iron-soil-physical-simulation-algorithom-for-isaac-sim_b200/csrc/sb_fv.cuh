@@ -37,6 +37,11 @@ struct FvConst {
   int ny, nx, pitch, tiles_x, nblocks;  // FX: tiles_x = column strips, nblocks = launch grid
   int rows_per_warp;                    // batched strips: rows of one warp's strip
   int row_chunks;                       // FX streaming kernel: row chunks per strip
+  // persistent substep loop: rows of a chunk, and its blocks of block_rows rows
+  // (chunk_blocks of them, the last one may be shorter) whose wet flags are kept
+  // in wet[buffer][strip][chunk * chunk_blocks + block]
+  int chunk_rows, block_rows, chunk_blocks;
+  int* wet;
   double dx, dy, K, g, cfl, dry, mu_g, c_half, kg, min_spacing;
   // fixed-point constants
   double Q;
@@ -70,6 +75,8 @@ struct FvControl {
   // persistent substep loop: substep k's wave-speed maximum goes to slot
   // k % 3 (cleared two substeps ahead by the barrier)
   unsigned long long wave3[3];
+  int wetn[3];  // likewise: blocks that the substep left wet
+  int pad3;
 };
 
 // Ledger record layout (filled by the ledger kernels of sb_ledger.cuh).
@@ -182,8 +189,9 @@ __device__ __forceinline__ float fx_friction(float dec, float spd) {
 // tangential momentum components.  Outputs: mass flux (quanta or raw),
 // normal-momentum flux seen by L (minus) and by R (plus), tangential flux.
 // --------------------------------------------------------------------------
-// FX face: un/ut are the cells' velocity components q/h (0 for empty cells), cl/cr
-// their celerities sqrt(K g h).  The hydrostatic depth only differs from h on
+// FX face: hl/hr are the cells' depths in metres (h quanta * Q), un/ut their
+// velocity components q/h (0 for empty cells), cl/cr their celerities
+// sqrt(K g h).  The hydrostatic depth only differs from h on
 // the lower side of a face (d > 0): it and its celerity are computed once, for
 // whichever side is lower, and selected (on a flat face the same expressions
 // reproduce h and the prepared celerity exactly), so the face has no branch
@@ -193,9 +201,9 @@ __device__ __forceinline__ float fx_friction(float dec, float spd) {
 // and reciprocals go through fx_sqrt / fx_rcp (IEEE when FAST is false).
 template <bool FAST = false>
 __device__ __forceinline__ void face_fx(const FvConst& c, float lam, int bl, int br, int hlq,
-                                        int hrq, float unl, float utl, float unr, float utr,
-                                        float cl, float cr, int& m, float& fnm, float& fnp,
-                                        float& ft) {
+                                        int hrq, float hl, float hr, float unl, float utl,
+                                        float unr, float utr, float cl, float cr, int& m,
+                                        float& fnm, float& fnp, float& ft) {
   if ((hlq | hrq) == 0) {
     // both cells empty: every flux below is a (signed) zero; return +0 (the
     // sign of a zero flux never changes a field value)
@@ -203,15 +211,11 @@ __device__ __forceinline__ void face_fx(const FvConst& c, float lam, int bl, int
     fnm = fnp = ft = 0.f;
     return;
   }
-  const int bface = max(bl, br);
-  const int dl = bface - bl;
-  const int dr = bface - br;
-  const float hl = (float)hlq * c.Qf;
-  const float hr = (float)hrq * c.Qf;
   // only the lower side of a face can have a hydrostatic depth below h
-  const bool llow = dl != 0;
+  const bool llow = br > bl;
+  const int step = llow ? br - bl : bl - br;
   const float hlow = llow ? hl : hr;
-  const float hs_low = fmaxf(hlow - (float)(dl + dr) * c.QKf, 0.f);
+  const float hs_low = fmaxf(hlow - (float)step * c.QKf, 0.f);
   const float cs_low = fx_sqrt<FAST>(c.KGf * hs_low);
   const float cor_low = (c.HKGf * hlow) * hlow - (c.HKGf * hs_low) * hs_low;
   const float hsl = llow ? hs_low : hl, csl = llow ? cs_low : cl, corl = llow ? cor_low : 0.f;
@@ -229,9 +233,8 @@ __device__ __forceinline__ void face_fx(const FvConst& c, float lam, int bl, int
   const float fh = 0.5f * (qnsl + qnsr) - half * (hsr - hsl);
   const float fn = 0.5f * (fnl + fnr) - half * (qnsr - qnsl);
   ft = 0.5f * (ftl + ftr) - half * (qtsr - qtsl);
-  float mf = rintf((lam * fh) * c.invQf);
-  mf = fminf(fmaxf(mf, -1073741824.f), 1073741824.f);
-  int mi = (int)mf;
+  // rounded to nearest; the conversion saturates, far beyond the donor's limit
+  int mi = __float2int_rn((lam * fh) * c.invQf);
   mi = mi > 0 ? min(mi, hlq >> 2) : max(mi, -(hrq >> 2));
   m = mi;
   fnm = fn + corl;
@@ -467,11 +470,13 @@ __global__ void __launch_bounds__(kThreads)
       float fnm = 0.f, fnp = 0.f, ft = 0.f;
       if (valid) {
         if (east)
-          face_fx(c, lamx_f, s.b[la], s.b[lb], s.h[la], s.h[lb], s.u[la], s.v[la], s.u[lb],
-                  s.v[lb], s.cel[la], s.cel[lb], m, fnm, fnp, ft);
+          face_fx(c, lamx_f, s.b[la], s.b[lb], s.h[la], s.h[lb], (float)s.h[la] * c.Qf,
+                  (float)s.h[lb] * c.Qf, s.u[la], s.v[la], s.u[lb], s.v[lb], s.cel[la],
+                  s.cel[lb], m, fnm, fnp, ft);
         else
-          face_fx(c, lamy_f, s.b[la], s.b[lb], s.h[la], s.h[lb], s.v[la], s.u[la], s.v[lb],
-                  s.u[lb], s.cel[la], s.cel[lb], m, fnm, fnp, ft);
+          face_fx(c, lamy_f, s.b[la], s.b[lb], s.h[la], s.h[lb], (float)s.h[la] * c.Qf,
+                  (float)s.h[lb] * c.Qf, s.v[la], s.u[la], s.v[lb], s.u[lb], s.cel[la],
+                  s.cel[lb], m, fnm, fnp, ft);
       }
       if (east) {
         s.em[f] = m; s.enm[f] = fnm; s.enp[f] = fnp; s.et[f] = ft;
@@ -647,7 +652,7 @@ constexpr int kMinChunkRows = 5;  // shortest row chunk of one strip warp (701^2
 
 struct FxCell {
   int b, h;
-  float qx, qy, u, v, cel;
+  float qx, qy, hf, u, v, cel;  // hf: depth in metres
 };
 
 // CG = false: read-only-cache loads (fields written by an earlier launch);
@@ -660,7 +665,9 @@ __device__ __forceinline__ void fx_load(const FvConst& c, const int32_t* __restr
                                         const float* __restrict__ qy, int row, int gx, bool colok,
                                         FxCell& x) {
   if (colok && row >= 0 && row < c.ny) {
-    const size_t gi = (size_t)row * c.pitch + gx;
+    // 32-bit offsets (one address instruction per access): a context's buffers
+    // hold over 200 bytes per cell, so a grid has far fewer than 2^32 of them
+    const unsigned gi = (unsigned)row * (unsigned)c.pitch + (unsigned)gx;
     x.b = __ldg(b + gi);  // the support does not change during a substep loop
     if constexpr (CG) {
       x.h = __ldcg(h + gi);
@@ -682,12 +689,12 @@ __device__ __forceinline__ void fx_load(const FvConst& c, const int32_t* __restr
 // Per-cell velocity q/h (0 for an empty cell) and celerity sqrt(K g h).
 template <bool FAST>
 __device__ __forceinline__ void fx_prepare(const FvConst& c, FxCell& x) {
+  x.hf = (float)x.h * c.Qf;
   if (x.h > 0) {
-    const float hf = (float)x.h * c.Qf;
-    const float inv = fx_rcp<FAST>(hf);
+    const float inv = fx_rcp<FAST>(x.hf);
     x.u = x.qx * inv;
     x.v = x.qy * inv;
-    x.cel = fx_sqrt<FAST>(c.KGf * hf);
+    x.cel = fx_sqrt<FAST>(c.KGf * x.hf);
   } else {  // empty cell (the same values: q * 0 and sqrt(0)); no reciprocal or root
     x.u = x.qx * 0.f;
     x.v = x.qy * 0.f;
@@ -697,10 +704,12 @@ __device__ __forceinline__ void fx_prepare(const FvConst& c, FxCell& x) {
 
 // One warp's strip: columns strip*30-1 .. strip*30+30, rows y0 .. y1-1
 // of a grid whose row 0 starts at the given field pointers (row pitch
-// c.pitch).  Accumulates the impulse/energy sums into acc and the largest
-// next-substep wave speed into wave.  Every lane of the warp must call it.
-template <bool FAST = false, bool CG = false>
-__device__ __forceinline__ void fx_strip_run(const FvConst& c, const int32_t* __restrict__ bsrc,
+// c.pitch).  Accumulates this lane's impulse/energy sums into fa and the largest
+// next-substep wave speed into fwave.  Every lane of the warp must call it.
+// FLAGS: returns whether the new state of these rows of the strip holds any depth
+// or momentum.
+template <bool FAST = false, bool CG = false, bool FLAGS = false>
+__device__ __forceinline__ bool fx_strip_run(const FvConst& c, const int32_t* __restrict__ bsrc,
                                              const int32_t* __restrict__ hsrc,
                                              const float* __restrict__ qxsrc,
                                              const float* __restrict__ qysrc,
@@ -708,7 +717,7 @@ __device__ __forceinline__ void fx_strip_run(const FvConst& c, const int32_t* __
                                              float* __restrict__ qydst,
                                              const float* __restrict__ ext_x,
                                              const float* __restrict__ ext_y, int strip, int y0,
-                                             int y1, double sub_dt, double* acc, double& wave) {
+                                             int y1, double sub_dt, float* fa, float& fwave) {
   const int lane = threadIdx.x & 31;
   const int gx = strip * kStripOut - 1 + lane;
   const bool colok = gx >= 0 && gx < c.nx;
@@ -718,9 +727,7 @@ __device__ __forceinline__ void fx_strip_run(const FvConst& c, const int32_t* __
   const float lamy_f = (float)(sub_dt / c.dy);
   const float dtf = (float)sub_dt;
   const float dec = (float)(c.mu_g * sub_dt);
-  if (y0 >= c.ny) return;  // warp-uniform
-  float fa[kFvDiag] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  float fwave = 0.f;
+  if (y0 >= c.ny) return false;  // warp-uniform
   FxCell cur, nxt, nn;
   fx_load<CG>(c, bsrc, hsrc, qxsrc, qysrc, y0, gx, colok, cur);
   fx_load<CG>(c, bsrc, hsrc, qxsrc, qysrc, y0 + 1, gx, colok, nxt);
@@ -734,24 +741,24 @@ __device__ __forceinline__ void fx_strip_run(const FvConst& c, const int32_t* __
     fx_prepare<FAST>(c, cur);
     if (y0 > 0 && colok) {
       float fnm;
-      face_fx<FAST>(c, lamy_f, prv.b, cur.b, prv.h, cur.h, prv.v, prv.u, cur.v, cur.u, prv.cel,
+      face_fx<FAST>(c, lamy_f, prv.b, cur.b, prv.h, cur.h, prv.hf, cur.hf, prv.v, prv.u, cur.v, cur.u, prv.cel,
               cur.cel, ms, fnm, nnps, nts);
     }
   }
   fx_prepare<FAST>(c, nxt);
-#pragma unroll 2
-  for (int r = y0; r < y1; ++r) {
+  auto row = [&](int r, int& nz) {
     fx_load<CG>(c, bsrc, hsrc, qxsrc, qysrc, r + 2, gx, colok, nn);
     // east face: this column and the next lane's
     const int eb = __shfl_down_sync(0xffffffffu, cur.b, 1);
     const int eh = __shfl_down_sync(0xffffffffu, cur.h, 1);
+    const float ehf = __shfl_down_sync(0xffffffffu, cur.hf, 1);
     const float eu = __shfl_down_sync(0xffffffffu, cur.u, 1);
     const float ev = __shfl_down_sync(0xffffffffu, cur.v, 1);
     const float ec = __shfl_down_sync(0xffffffffu, cur.cel, 1);
     int me = 0;
     float enm = 0.f, enp = 0.f, et = 0.f;
     if (east_ok)
-      face_fx<FAST>(c, lamx_f, cur.b, eb, cur.h, eh, cur.u, cur.v, eu, ev, cur.cel, ec, me, enm, enp,
+      face_fx<FAST>(c, lamx_f, cur.b, eb, cur.h, eh, cur.hf, ehf, cur.u, cur.v, eu, ev, cur.cel, ec, me, enm, enp,
               et);
     // west face = the previous lane's east face
     const int mw = __shfl_up_sync(0xffffffffu, me, 1);
@@ -761,15 +768,10 @@ __device__ __forceinline__ void fx_strip_run(const FvConst& c, const int32_t* __
     int mn = 0;
     float nnm = 0.f, nnp = 0.f, nt = 0.f;
     if (colok && r + 1 < c.ny)
-      face_fx<FAST>(c, lamy_f, cur.b, nxt.b, cur.h, nxt.h, cur.v, cur.u, nxt.v, nxt.u, cur.cel,
+      face_fx<FAST>(c, lamy_f, cur.b, nxt.b, cur.h, nxt.h, cur.hf, nxt.hf, cur.v, cur.u, nxt.v, nxt.u, cur.cel,
               nxt.cel, mn, nnm, nnp, nt);
     if (out_lane) {
-      const size_t gi = (size_t)r * c.pitch + gx;
-      float ax = 0.f, ay = 0.f;
-      if (c.has_external) {
-        ax = ext_x[gi];
-        ay = ext_y[gi];
-      }
+      const unsigned gi = (unsigned)r * (unsigned)c.pitch + (unsigned)gx;
       const int dh = ((0 - me + mw) - mn) + ms;
       const int hq = cur.h + dh;
       const float zero = 0.f;
@@ -779,20 +781,19 @@ __device__ __forceinline__ void fx_strip_run(const FvConst& c, const int32_t* __
       const bool wet = hn > c.dryf;
       const float qxn = wet ? cur.qx + dqx : 0.f;
       const float qyn = wet ? cur.qy + dqy : 0.f;
-      float vbx = 0.f, vby = 0.f, qex = qxn, qey = qyn, vex = 0.f, vey = 0.f;
-      if (wet) {
-        const float inv = fx_rcp<FAST>(hn);
-        vbx = qxn * inv;
-        vby = qyn * inv;
-        if (c.has_external) {
+      const float inv = wet ? fx_rcp<FAST>(hn) : 0.f;  // dry: zero momentum, zero velocity
+      float qex = qxn, qey = qyn, vex = qxn * inv, vey = qyn * inv;
+      if (c.has_external) {
+        const float ax = ext_x[gi], ay = ext_y[gi], vbx = vex, vby = vey;
+        if (wet) {
           qex = qxn + (hn * ax) * dtf;
           qey = qyn + (hn * ay) * dtf;
           vex = qex * inv;
           vey = qey * inv;
-        } else {
-          vex = vbx;
-          vey = vby;
         }
+        fa[2] += qex - qxn;
+        fa[3] += qey - qyn;
+        fa[7] += (hn * ((0.5f * (vbx + vex)) * ax + (0.5f * (vby + vey)) * ay)) * dtf;
       }
       const float spd = fx_sqrt<FAST>(vex * vex + vey * vey);
       const float fac = fx_friction<FAST>(dec, spd);
@@ -801,18 +802,15 @@ __device__ __forceinline__ void fx_strip_run(const FvConst& c, const int32_t* __
       hdst[gi] = hq;
       qxdst[gi] = qxo;
       qydst[gi] = qyo;
+      if constexpr (FLAGS) nz |= hq | __float_as_int(qxo) | __float_as_int(qyo);
       // per-lane diagnostics in float over this strip (one cell per row of
       // the chunk), folded into the double sums once at the end
       fa[0] += qxn - cur.qx;
       fa[1] += qyn - cur.qy;
-      fa[2] += qex - qxn;
-      fa[3] += qey - qyn;
       fa[4] += qxo - qex;
       fa[5] += qyo - qey;
       // friction dissipation 0.5 h (|v|^2 - |v fac|^2) = 0.5 h |v|^2 (1 - fac)(1 + fac)
       fa[6] += ((0.5f * hn) * (spd * spd)) * ((1.f - fac) * (1.f + fac));
-      if (c.has_external)
-        fa[7] += (hn * ((0.5f * (vbx + vex)) * ax + (0.5f * (vby + vey)) * ay)) * dtf;
       const float wv = spd * fac + fx_sqrt<FAST>(c.KGf * hn);  // |new velocity| + celerity
       fwave = fmaxf(fwave, wv);
     }
@@ -822,10 +820,11 @@ __device__ __forceinline__ void fx_strip_run(const FvConst& c, const int32_t* __
     cur = nxt;
     nxt = nn;
     fx_prepare<FAST>(c, nxt);
-  }
-#pragma unroll
-  for (int k = 0; k < kFvDiag; ++k) acc[k] += (double)fa[k];
-  wave = fmax(wave, (double)fwave);
+  };
+  int nz = 0;
+#pragma unroll 2
+  for (int r = y0; r < y1; ++r) row(r, nz);
+  return FLAGS && __any_sync(0xffffffffu, nz != 0);
 }
 
 template <bool FAST>
@@ -842,17 +841,17 @@ __global__ void __launch_bounds__(kThreads, 4)
   const int parity = ctl->parity;
   const int gw = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   double acc[kFvDiag];
-#pragma unroll
-  for (int k = 0; k < kFvDiag; ++k) acc[k] = 0.0;
-  double wave = 0.0;
+  float fa[kFvDiag] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, fwave = 0.f;
   // row chunk j of the strip: rows [j*ny/J, (j+1)*ny/J), balanced to within one row
   const int j = gw / c.tiles_x, nchunk = c.row_chunks;
   const int y0 = j < nchunk ? (int)((long long)j * c.ny / nchunk) : c.ny;
   const int y1 = j < nchunk ? (int)((long long)(j + 1) * c.ny / nchunk) : c.ny;
   fx_strip_run<FAST>(c, bsrc, parity ? h1 : h0, parity ? qx1 : qx0, parity ? qy1 : qy0,
                parity ? h0 : h1, parity ? qx0 : qx1, parity ? qy0 : qy1, ext_x, ext_y,
-               gw % c.tiles_x, y0, y1, sub_dt, acc, wave);
-  fv_finish(c, ctl, diag_acc, acc, wave, 0, &flag, sub_dt, parity, loop_handle, use_handle);
+               gw % c.tiles_x, y0, y1, sub_dt, fa, fwave);
+#pragma unroll
+  for (int k = 0; k < kFvDiag; ++k) acc[k] = (double)fa[k];
+  fv_finish(c, ctl, diag_acc, acc, (double)fwave, 0, &flag, sub_dt, parity, loop_handle, use_handle);
 }
 
 // --------------------------------------------------------------------------
@@ -864,12 +863,31 @@ __global__ void __launch_bounds__(kThreads, 4)
 // CTA sent by atomicMax) and releases the others by bumping a generation
 // word.  The impulse/energy sums stay in each lane's registers across the
 // substeps and are folded once per step, so a substep ends with one warp
-// maximum and one atomic per CTA.  Field loads in the loop are L2-coherent
+// maximum and one atomic per CTA.
+//
+// Dry ground is skipped.  The before-step ledger, which reads every cell, flags
+// the blocks that hold any depth or momentum; a block whose 3x3 neighbourhood of
+// blocks is dry stays dry (all its faces lie between empty cells), so it is
+// neither read nor written, except that its place in the other buffer is
+// cleared when its flag says that it holds something else.  Each substep leaves
+// the flags of what it wrote.
+// A chunk that is wet throughout, with its surroundings, is one run of its own
+// warp, and so is every run of wet blocks while most of the grid is wet (a block
+// of its own costs an extra row's face and flags of other chunks to read: 7 % at
+// 4096^2 wet everywhere).  Else the wet blocks are taken by warps of different
+// SMs, because the rows of a strip are a chain of L2 latencies (about 0.7 us
+// each for a warp alone; 121 rows of a chunk took 90 us of a substep).
+// 4096^2 site with 21 k wet cells: 41 us per substep (135 before), of which 37 are
+// one or two wet blocks of 16 rows in a row.  701^2 with 360 wet cells: 12.4 us
+// (13.0), launch, barrier and one chunk of 5 rows.
+//
+// Field loads in the loop are L2-coherent
 // (the previous substep's writes come from other CTAs of this launch).  The
 // barrier wait is bounded: after kFvBarrierPolls polls the CTA records a wait
 // failure (SB_ERR_WAIT_LIMIT) and the loop ends.
 // --------------------------------------------------------------------------
 constexpr unsigned kFvBarrierPolls = 1u << 22;
+constexpr int kFvChunkBlocks = 8;  // most blocks of a chunk: 3 x (8 + 2) flags, one per lane
 
 template <bool FAST>
 __global__ void __launch_bounds__(kThreads, 4)
@@ -879,16 +897,29 @@ __global__ void __launch_bounds__(kThreads, 4)
                    FvControl* ctl, double* __restrict__ diag_acc) {
   __shared__ double fold[fold_words(kFvDiag)];
   __shared__ double wred[kThreads / 32];
+  __shared__ int nred[kThreads / 32];
   __shared__ unsigned s_gen;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gw = blockIdx.x * (kThreads / 32) + warp;
-  const int j = gw / c.tiles_x, nchunk = c.row_chunks;
-  const int y0 = j < nchunk ? (int)((long long)j * c.ny / nchunk) : c.ny;
-  const int y1 = j < nchunk ? (int)((long long)(j + 1) * c.ny / nchunk) : c.ny;
-  const int strip = gw % c.tiles_x;
-  double acc[kFvDiag];
+  const int j = gw / c.tiles_x, strip = gw % c.tiles_x;
+  const int y0 = min(j * c.chunk_rows, c.ny), y1 = min(y0 + c.chunk_rows, c.ny);
+  const int blocks = (y1 - y0 + c.block_rows - 1) / c.block_rows;  // 0: a spare warp
+  const int column = c.row_chunks * c.chunk_blocks;  // blocks of a strip
+  const int own = strip * column + j * c.chunk_blocks;
+  // the chunk whose block t this warp takes: its own for t = 0, else far away, so
+  // that the blocks of a partly wet chunk go to warps of different SMs
+  const int chunks = c.tiles_x * c.row_chunks, apart = max(1, chunks / c.chunk_blocks);
+  auto chunk_of = [&](int t) {
+    int q = gw + t * apart;
+    while (q >= chunks) q -= chunks;  // once, or a few times with fewer chunks than blocks
+    return q;
+  };
+  __shared__ unsigned near[kThreads / 32][kFvChunkBlocks];
+  // this thread's sums over the step's substeps; in shared memory, they leave 16
+  // registers to the strip
+  __shared__ double sums[kFvDiag][kThreads];
 #pragma unroll
-  for (int k = 0; k < kFvDiag; ++k) acc[k] = 0.0;
+  for (int k = 0; k < kFvDiag; ++k) sums[k][threadIdx.x] = 0.0;
   // The loop control (remaining time, dt, parity, substep count) is the same
   // arithmetic in every CTA, so each CTA keeps its own copy in shared memory
   // (thread 0 advances it): a barrier needs one wave-speed maximum (slot
@@ -897,6 +928,7 @@ __global__ void __launch_bounds__(kThreads, 4)
   struct LoopCtl {
     double remaining, sub_dt, max_cfl, wave;
     int parity, substeps, cfl_limited, status, done;
+    int dense;  // the last substep left at least half of the blocks wet
   };
   __shared__ LoopCtl L;
   if (threadIdx.x == 0) {
@@ -909,18 +941,91 @@ __global__ void __launch_bounds__(kThreads, 4)
     L.cfl_limited = *(volatile int*)&ctl->cfl_limited;
     L.status = *(volatile int*)&ctl->status;
     L.done = *(volatile int*)&ctl->done;
+    L.dense = 0;
   }
   __syncthreads();
   for (int k = 0; !L.done; ++k) {
     const double sub_dt = L.sub_dt;
     const int parity = L.parity;
     if (threadIdx.x == 0) s_gen = *(volatile unsigned*)&ctl->gen;
-    double wave = 0.0;
-    fx_strip_run<FAST, true>(c, bsrc, parity ? h1 : h0, parity ? qx1 : qx0, parity ? qy1 : qy0,
-                             parity ? h0 : h1, parity ? qx0 : qx1, parity ? qy0 : qy1, ext_x,
-                             ext_y, strip, y0, y1, sub_dt, acc, wave);
+    float fa[kFvDiag] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, fwave = 0.f;
+    int wet_blocks = 0;
+    const bool dense = L.dense;
+    if (blocks > 0) {
+      const int size = c.tiles_x * column;
+      const int* wet = c.wet + parity * size;
+      int* next = c.wet + (parity ^ 1) * size;
+      int32_t* hdst = parity ? h0 : h1;
+      float *qxdst = parity ? qx0 : qx1, *qydst = parity ? qy0 : qy1;
+      // this warp's chunk (t = 0) and those whose block t it takes when they are
+      // only partly wet: bits 3 i .. 3 i + 8 of near[t] are the neighbourhood of
+      // block i (lanes: blocks -1 .. chunk_blocks by strips -1 .. 1), bit 31 that
+      // all of it is wet
+      const int shared = dense ? 1 : c.chunk_blocks;
+#pragma unroll
+      for (int t = 0; t < kFvChunkBlocks; ++t) {
+        if (t >= shared) break;
+        const int q = chunk_of(t), qj = q / c.tiles_x;
+        const int fi = lane / 3 - 1, fs = q - qj * c.tiles_x - 1 + lane % 3;
+        const bool in = fs >= 0 && fs < c.tiles_x &&
+                        (fi < 0                ? qj > 0
+                         : fi < c.chunk_blocks ? qj * c.chunk_rows + fi * c.block_rows < c.ny
+                                               : fi == c.chunk_blocks && qj + 1 < c.row_chunks);
+        const int f = in ? __ldcg(wet + fs * column + qj * c.chunk_blocks + fi) : 0;
+        unsigned m = __ballot_sync(0xffffffffu, f != 0);
+        if (__all_sync(0xffffffffu, f || !in)) m |= 0x80000000u;
+        if (lane == 0) near[warp][t] = m;
+      }
+      const unsigned stale =
+          __ballot_sync(0xffffffffu, lane < blocks && __ldcg(next + own + lane) != 0);
+      __syncwarp();
+      for (int i = 0; i < blocks; ++i) {
+        // dry, and the other buffer is not
+        if ((near[warp][0] >> (3 * i)) & 0x1ffu || !((stale >> i) & 1u)) continue;
+        const int gx = strip * kStripOut - 1 + lane, r0 = y0 + i * c.block_rows;
+        if (lane >= 1 && lane <= kStripOut && gx < c.nx)
+          for (int r = r0; r < min(r0 + c.block_rows, y1); ++r) {
+            const size_t gi = (size_t)r * c.pitch + gx;
+            hdst[gi] = 0;
+            qxdst[gi] = 0.f;
+            qydst[gi] = 0.f;
+          }
+        if (lane == 0) next[own + i] = 0;
+      }
+      for (int t = 0; t < shared; ++t) {
+        const unsigned m = near[warp][t];
+        // runs of wet blocks of the own chunk where it is wet throughout or most of
+        // the grid is; else single blocks, shared out
+        const bool runs = dense || (m >> 31);
+        if (runs && t > 0) continue;
+        const int q = chunk_of(t), qj = q / c.tiles_x, qs = q - qj * c.tiles_x;
+        const int q0 = qj * c.chunk_rows, q1 = min(q0 + c.chunk_rows, c.ny);
+        const int end = runs ? blocks : t + 1;
+        for (int i = runs ? 0 : t; i < end;) {
+          int e = i + 1;
+          if (!((m >> (3 * i)) & 0x1ffu) || q0 + i * c.block_rows >= q1) {
+            i = e;
+            continue;
+          }
+          while (e < end && ((m >> (3 * e)) & 0x1ffu)) ++e;
+          const bool nz = fx_strip_run<FAST, true, true>(
+              c, bsrc, parity ? h1 : h0, parity ? qx1 : qx0, parity ? qy1 : qy0, hdst, qxdst,
+              qydst, ext_x, ext_y, qs, q0 + i * c.block_rows, min(q0 + e * c.block_rows, q1),
+              sub_dt, fa, fwave);
+          if (lane < e - i) next[qs * column + qj * c.chunk_blocks + i + lane] = nz;
+          if (nz) wet_blocks += e - i;
+          i = e;
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kFvDiag; ++q) sums[q][threadIdx.x] += (double)fa[q];
+    double wave = (double)fwave;
     wave = warp_max(wave);
-    if (lane == 0) wred[warp] = wave;
+    if (lane == 0) {
+      wred[warp] = wave;
+      nred[warp] = wet_blocks;
+    }
     // the CTA barrier orders every thread's field writes before thread 0's
     // device-scope fence and arrival (the grid-barrier pattern: one fence)
     __syncthreads();
@@ -929,12 +1034,17 @@ __global__ void __launch_bounds__(kThreads, 4)
 #pragma unroll
       for (int w = 0; w < kThreads / 32; ++w) m = fmax(m, wred[w]);
       atomicMax(&ctl->wave3[k % 3], (unsigned long long)__double_as_longlong(m));
+      int n = 0;
+#pragma unroll
+      for (int w = 0; w < kThreads / 32; ++w) n += nred[w];
+      if (n) atomicAdd(&ctl->wetn[k % 3], n);
       __threadfence();
       const unsigned prev = atomicAdd(&ctl->arrive, 1u);
       bool failed = false;
       if (prev == gridDim.x - 1) {
         ctl->arrive = 0;
         ctl->wave3[(k + 1) % 3] = 0ull;  // read by every CTA two barriers ago
+        ctl->wetn[(k + 1) % 3] = 0;
         __threadfence();
         atomicAdd(&ctl->gen, 1u);  // release
       } else {
@@ -959,6 +1069,7 @@ __global__ void __launch_bounds__(kThreads, 4)
       } else {
         const double w = __longlong_as_double((long long)__ldcg(&ctl->wave3[k % 3]));
         L.wave = w;
+        L.dense = 2 * (long long)__ldcg(&ctl->wetn[k % 3]) >= (long long)c.tiles_x * column;
         if (!(L.remaining > 1.0e-14)) {
           L.done = 1;
         } else if (L.substeps >= c.max_substeps) {
@@ -976,6 +1087,14 @@ __global__ void __launch_bounds__(kThreads, 4)
     }
     __syncthreads();
   }
+  // The current buffer's flags are cleared for the next step's ledger; the other
+  // buffer, which only this kernel writes, keeps its flags (all set if a wait
+  // gave up: its contents are unknown then).
+  if (lane < blocks) {
+    const int size = c.tiles_x * column;
+    c.wet[L.parity * size + own + lane] = 0;
+    if (L.status == 6) c.wet[(L.parity ^ 1) * size + own + lane] = 1;
+  }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     // every CTA holds the same loop control; one writes it back
     ctl->remaining = L.remaining;
@@ -989,6 +1108,9 @@ __global__ void __launch_bounds__(kThreads, 4)
     ctl->done = 1;
   }
   // the step's impulse/energy sums of this CTA, once
+  double acc[kFvDiag];
+#pragma unroll
+  for (int k = 0; k < kFvDiag; ++k) acc[k] = sums[k][threadIdx.x];
   const double* bt = block_fold<double, kFvDiag, kFvDiag>(acc, fold);
   if (threadIdx.x < kFvDiag) {
     double* a = diag_acc + (size_t)threadIdx.x * c.nblocks + blockIdx.x;

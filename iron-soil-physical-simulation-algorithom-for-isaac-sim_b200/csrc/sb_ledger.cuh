@@ -43,8 +43,8 @@ __device__ __forceinline__ void ledger_cell_fx(const FvConst& c, const int32_t* 
                                                const float* __restrict__ qy,
                                                const float* __restrict__ ext_x,
                                                const float* __restrict__ ext_y, double datum,
-                                               int r, int col, double* v, long long& iq0,
-                                               long long& iq1, long long& iq2) {
+                                               int r, int col, int* wet, double* v,
+                                               long long& iq0, long long& iq1, long long& iq2) {
   const size_t gi = (size_t)r * c.pitch + col;
   const int w6 = vertex_weight6(r, col, c.ny, c.nx);
   const int hq = h[gi], bq = b[gi], zq = z[gi];
@@ -58,6 +58,11 @@ __device__ __forceinline__ void ledger_cell_fx(const FvConst& c, const int32_t* 
   const double hv = (double)hq * c.Q;
   v[L_NEGMINH] = fmax(v[L_NEGMINH], -hv);
   if (hq == 0 && qxf == 0.f && qyf == 0.f) return;
+  if (wet) {  // the substep loop's block of this cell is not dry
+    const int j = r / c.chunk_rows;
+    wet[((col / kStripOut) * c.row_chunks + j) * c.chunk_blocks +
+        (r - j * c.chunk_rows) / c.block_rows] = 1;
+  }
   const double bv = (double)bq * c.Q + datum;
   const double qxv = (double)qxf, qyv = (double)qyf;
   iq0 += hq;
@@ -104,10 +109,10 @@ __device__ __forceinline__ void ledger_cell(const FvConst& c,
                                             const typename FvTypes<FX>::R* __restrict__ qy,
                                             const typename FvTypes<FX>::R* __restrict__ ext_x,
                                             const typename FvTypes<FX>::R* __restrict__ ext_y,
-                                            double datum, int r, int col, double* v,
+                                            double datum, int r, int col, int* wet, double* v,
                                             long long& iq0, long long& iq1, long long& iq2) {
   if constexpr (FX) {
-    ledger_cell_fx(c, b, z, h, qx, qy, ext_x, ext_y, datum, r, col, v, iq0, iq1, iq2);
+    ledger_cell_fx(c, b, z, h, qx, qy, ext_x, ext_y, datum, r, col, wet, v, iq0, iq1, iq2);
   } else {
     const size_t gi = (size_t)r * c.pitch + col;
     const int w6 = vertex_weight6(r, col, c.ny, c.nx);
@@ -257,6 +262,10 @@ __global__ void __launch_bounds__(kThreads, 3)
   for (int k = 0; k < L_NP; ++k) v[k] = 0.0;
   v[L_NEGMINH] = -1.0e300;
   long long iq0 = 0, iq1 = 0, iq2 = 0;
+  // a before-step ledger flags the wet blocks of the current buffer
+  int* wet = mode == 0 && c.wet
+                 ? c.wet + parity * c.tiles_x * c.row_chunks * c.chunk_blocks
+                 : nullptr;
   {
     // warp items = 32-column segments of one row; a lane owns one column
     const int strips = (c.nx + 31) >> 5;
@@ -270,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     for (; it < items; it += nwarps) {
       const int col = (s << 5) + lane;
       if (col < c.nx)
-        ledger_cell<FX>(c, b, z, h, qx, qy, ext_x, ext_y, datum, r, col, v, iq0, iq1, iq2);
+        ledger_cell<FX>(c, b, z, h, qx, qy, ext_x, ext_y, datum, r, col, wet, v, iq0, iq1, iq2);
       r += dr;
       s += ds;
       if (s >= strips) {
@@ -355,7 +364,10 @@ __device__ __forceinline__ void fv_begin_body(FvControl* ctl, const double* dt) 
     ctl->static_skip = 0;
     ctl->arrive = 0;
     ctl->wait_fail = 0;
-    for (int k = 0; k < 3; ++k) ctl->wave3[k] = 0ull;
+    for (int k = 0; k < 3; ++k) {
+      ctl->wave3[k] = 0ull;
+      ctl->wetn[k] = 0;
+    }
   }
 }
 

@@ -156,6 +156,8 @@ struct sb_ctx {
   int fv_exact = 0;  // 1: FX32 strip kernel with the CPU mirror's IEEE arithmetic
   int fv_persistent = 0;  // 1: step graphs run the substeps in one cooperative launch
   int fv_rows = 0;  // FX streaming kernel: row chunks per strip
+  int fv_chunk_rows = 0, fv_block_rows = 0, fv_chunk_blocks = 0;  // see FvConst
+  int* fv_wet = nullptr;
   int fv_strips = 0;
   int fv_stream_blocks = 0;
   int ledger_blocks = 0;
@@ -334,6 +336,12 @@ FvConst make_const(const sb_ctx* ctx, const sb_mobile_params* p) {
     c.tiles_x = ctx->fv_strips;
     c.nblocks = ctx->fv_stream_blocks;
     c.row_chunks = ctx->fv_rows;
+    if (ctx->fv_persistent) {
+      c.chunk_rows = ctx->fv_chunk_rows;
+      c.block_rows = ctx->fv_block_rows;
+      c.chunk_blocks = ctx->fv_chunk_blocks;
+      c.wet = ctx->fv_wet;
+    }
   }
   c.dx = ctx->d.dx_m;
   c.dy = ctx->d.dy_m;
@@ -753,19 +761,24 @@ int sb_ctx_create(const sb_grid_desc* desc, sb_ctx** out) {
     ctx->fv_strips = (d.nx + kStripOut - 1) / kStripOut;
     // row chunks per strip: at most one wave of warps (4 CTAs of 8 warps on
     // each SM of this device) and at least kMinChunkRows rows per chunk (every
-    // chunk pays one extra row of loads, two cell preparations and one face);
-    // the chunks split the rows evenly (sizes differ by at most one row)
+    // chunk pays one extra row of loads, two cell preparations and one face)
     int sms = 0;
     SB_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d.device));
-    const long long want_warps = (long long)std::max(sms, 1) * 32;
-    long long chunks = want_warps / ctx->fv_strips;
-    chunks = std::min<long long>(chunks, d.ny / kMinChunkRows);
-    chunks = std::max<long long>(chunks, 1);
+    const long long most = std::max(1LL, std::max(sms, 1) * 32LL / ctx->fv_strips);
+    long long rows = std::max<long long>(kMinChunkRows, (d.ny + most - 1) / most);
     if (const char* rows_env = std::getenv("SOILB200_FV_ROWS")) {
       const long long r = std::atoll(rows_env);
-      if (r >= 1 && r <= 4096) chunks = (d.ny + r - 1) / r;
+      if (r >= 1 && r <= 4096) rows = r;
     }
+    const long long chunks = (d.ny + rows - 1) / rows;
     ctx->fv_rows = (int)chunks;
+    // wet flags for blocks of 16 rows (a chunk's neighbourhood is one warp read:
+    // at most 8 blocks)
+    ctx->fv_chunk_rows = (int)rows;
+    ctx->fv_block_rows = (int)std::min(rows, std::max(16LL, (rows + kFvChunkBlocks - 1) / kFvChunkBlocks));
+    ctx->fv_chunk_blocks = (int)((rows + ctx->fv_block_rows - 1) / ctx->fv_block_rows);
+    dev.add(&ctx->fv_wet,
+            (size_t)2 * ctx->fv_strips * chunks * ctx->fv_chunk_blocks * sizeof(int));
     const long long warps = (long long)ctx->fv_strips * chunks;
     ctx->fv_stream_blocks = (int)((warps + kThreads / 32 - 1) / (kThreads / 32));
     // the persistent substep loop needs every CTA resident at once
