@@ -45,7 +45,8 @@ __global__ void batch_begin_kernel(int npatch, BatchCtl* ctl, const double* dt) 
 __global__ void __launch_bounds__(kThreads)
     batch_ledger_kernel(const BatchPatch* __restrict__ patches, const int* __restrict__ band_patch,
                         int nbands, BatchArena a, const BatchCtl* __restrict__ ctl,
-                        double* __restrict__ partials, long long* __restrict__ ipartials) {
+                        double* __restrict__ partials, long long* __restrict__ ipartials,
+                        int mode) {
   __shared__ double fold[fold_words(L_NP)];
   const int band = blockIdx.x;
   if (band >= nbands) return;
@@ -56,17 +57,18 @@ __global__ void __launch_bounds__(kThreads)
   const long long base = P.base;
   const int r0 = (band - P.first_band) * kBandRows;
   const int r1 = min(r0 + kBandRows, c.ny);
+  LedgerScan scan(c, mode == 0, P.static_limit, nullptr, fold);
+  // a warp takes every eighth row of the band
+  const int lane = threadIdx.x & 31;
+  for (int r = r0 + (threadIdx.x >> 5); r < r1; r += kThreads / 32)
+    for (int col = 0; col < c.nx; col += kLedgerCols)
+      ledger_quad_fx<false>(c, a.b + base, a.z + base, a.h[parity] + base, a.qx[parity] + base,
+                            a.qy[parity] + base, nullptr, nullptr, P.datum, r,
+                            col + lane * kLedgerQuad, scan);
   double v[L_NP];
-#pragma unroll
-  for (int k = 0; k < L_NP; ++k) v[k] = 0.0;
-  v[L_NEGMINH] = -1.0e300;
-  long long iq0 = 0, iq1 = 0, iq2 = 0;
-  const int n = (r1 - r0) * c.nx;
-  for (int i = threadIdx.x; i < n; i += kThreads)
-    ledger_cell<true>(c, a.b + base, a.z + base, a.h[parity] + base, a.qx[parity] + base,
-                      a.qy[parity] + base, nullptr, nullptr, P.datum, r0 + i / c.nx, i % c.nx, nullptr, v,
-                      iq0, iq1, iq2);
-  ledger_block_store(v, iq0, iq1, iq2, fold, partials + (size_t)band * L_NP,
+  long long iq[kLedgerI64];
+  scan.finish(c, v, iq);
+  ledger_block_store(v, iq, fold, partials + (size_t)band * L_NP,
                      ipartials + (size_t)band * kLedgerI64, 1);
 }
 

@@ -209,7 +209,7 @@ int batch_build_graph(sb_batch* bt) {
   }
   {
     void* args[] = {&bt->d_patches, &bt->d_band_patch, &nbands, &a, &bt->d_ctl,
-                    &bt->d_band_partials, &bt->d_band_ipartials};
+                    &bt->d_band_partials, &bt->d_band_ipartials, &mode0};
     if ((rc = badd_kernel(bt, g, &n1, &n0, 1, (void*)batch_ledger_kernel, gb, args))) return rc;
   }
   {
@@ -242,7 +242,7 @@ int batch_build_graph(sb_batch* bt) {
   SB_BCUDA(bt, cudaGraphAddEventRecordNode(&ne1, g, &nloop, 1, bt->ev[1]));
   {
     void* args[] = {&bt->d_patches, &bt->d_band_patch, &nbands, &a, &bt->d_ctl,
-                    &bt->d_band_partials, &bt->d_band_ipartials};
+                    &bt->d_band_partials, &bt->d_band_ipartials, &mode1};
     if ((rc = badd_kernel(bt, g, &n3, &ne1, 1, (void*)batch_ledger_kernel, gb, args))) return rc;
   }
   {

@@ -75,9 +75,24 @@ struct FvControl {
   // persistent substep loop: substep k's wave-speed maximum goes to slot
   // k % 3 (cleared two substeps ahead by the barrier)
   unsigned long long wave3[3];
-  int wetn[3];  // likewise: blocks that the substep left wet
+  // persistent substep loop: CTAs that arrived (low 32 bits) and the blocks that
+  // they left wet (high 32 bits); their total, for the substep's slot k % 3
+  unsigned long long arrive_wet;
+  int wetn[3];
+  // from the before-step ledger: its threads whose cells are mostly wet, and what
+  // that makes the first substep (LoopCtl.dense)
+  unsigned int wet_threads;
+  int dense;
   int pad3;
 };
+
+// How the persistent loop visits its blocks when n of all are wet.  2 (at least
+// 7/8): all of them, without waiting for a flag (at 1024^2, all wet, the flag loads
+// cost 1.2 of 23.8 us a substep); 1 (at least half): runs of wet blocks of the
+// warp's own chunk; 0: the wet blocks of partly wet chunks shared out among warps.
+__device__ __forceinline__ int fv_dense(long long n, long long all) {
+  return 8 * n >= 7 * all ? 2 : 2 * n >= all ? 1 : 0;
+}
 
 // Ledger record layout (filled by the ledger kernels of sb_ledger.cuh).
 enum LedgerSlot {
@@ -896,8 +911,8 @@ __global__ void __launch_bounds__(kThreads, 4)
                    const float* __restrict__ ext_x, const float* __restrict__ ext_y,
                    FvControl* ctl, double* __restrict__ diag_acc) {
   __shared__ double fold[fold_words(kFvDiag)];
-  __shared__ double wred[kThreads / 32];
-  __shared__ int nred[kThreads / 32];
+  // a warp's wave-speed maximum (float bits: not negative, never a NaN) and its wet blocks
+  __shared__ uint2 wred[kThreads / 32];
   __shared__ unsigned s_gen;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gw = blockIdx.x * (kThreads / 32) + warp;
@@ -906,6 +921,10 @@ __global__ void __launch_bounds__(kThreads, 4)
   const int blocks = (y1 - y0 + c.block_rows - 1) / c.block_rows;  // 0: a spare warp
   const int column = c.row_chunks * c.chunk_blocks;  // blocks of a strip
   const int own = strip * column + j * c.chunk_blocks;
+  const long long every =  // blocks with at least one row
+      (long long)c.tiles_x *
+      ((c.row_chunks - 1) * c.chunk_blocks +
+       (c.ny - (c.row_chunks - 1) * c.chunk_rows + c.block_rows - 1) / c.block_rows);
   // the chunk whose block t this warp takes: its own for t = 0, else far away, so
   // that the blocks of a partly wet chunk go to warps of different SMs
   const int chunks = c.tiles_x * c.row_chunks, apart = max(1, chunks / c.chunk_blocks);
@@ -928,7 +947,7 @@ __global__ void __launch_bounds__(kThreads, 4)
   struct LoopCtl {
     double remaining, sub_dt, max_cfl, wave;
     int parity, substeps, cfl_limited, status, done;
-    int dense;  // the last substep left at least half of the blocks wet
+    int dense;  // the last substep left at least half (1), 7/8 (2) of the blocks wet
   };
   __shared__ LoopCtl L;
   if (threadIdx.x == 0) {
@@ -941,7 +960,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     L.cfl_limited = *(volatile int*)&ctl->cfl_limited;
     L.status = *(volatile int*)&ctl->status;
     L.done = *(volatile int*)&ctl->done;
-    L.dense = 0;
+    L.dense = *(volatile int*)&ctl->dense;
   }
   __syncthreads();
   for (int k = 0; !L.done; ++k) {
@@ -950,7 +969,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     if (threadIdx.x == 0) s_gen = *(volatile unsigned*)&ctl->gen;
     float fa[kFvDiag] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, fwave = 0.f;
     int wet_blocks = 0;
-    const bool dense = L.dense;
+    const int dense = L.dense;
     if (blocks > 0) {
       const int size = c.tiles_x * column;
       const int* wet = c.wet + parity * size;
@@ -962,35 +981,40 @@ __global__ void __launch_bounds__(kThreads, 4)
       // block i (lanes: blocks -1 .. chunk_blocks by strips -1 .. 1), bit 31 that
       // all of it is wet
       const int shared = dense ? 1 : c.chunk_blocks;
+      if (dense == 2) {  // every block is visited: no flag is waited for
+        if (lane == 0) near[warp][0] = 0xffffffffu;
+        __syncwarp();
+      } else {
 #pragma unroll
-      for (int t = 0; t < kFvChunkBlocks; ++t) {
-        if (t >= shared) break;
-        const int q = chunk_of(t), qj = q / c.tiles_x;
-        const int fi = lane / 3 - 1, fs = q - qj * c.tiles_x - 1 + lane % 3;
-        const bool in = fs >= 0 && fs < c.tiles_x &&
-                        (fi < 0                ? qj > 0
-                         : fi < c.chunk_blocks ? qj * c.chunk_rows + fi * c.block_rows < c.ny
-                                               : fi == c.chunk_blocks && qj + 1 < c.row_chunks);
-        const int f = in ? __ldcg(wet + fs * column + qj * c.chunk_blocks + fi) : 0;
-        unsigned m = __ballot_sync(0xffffffffu, f != 0);
-        if (__all_sync(0xffffffffu, f || !in)) m |= 0x80000000u;
-        if (lane == 0) near[warp][t] = m;
-      }
-      const unsigned stale =
-          __ballot_sync(0xffffffffu, lane < blocks && __ldcg(next + own + lane) != 0);
-      __syncwarp();
-      for (int i = 0; i < blocks; ++i) {
-        // dry, and the other buffer is not
-        if ((near[warp][0] >> (3 * i)) & 0x1ffu || !((stale >> i) & 1u)) continue;
-        const int gx = strip * kStripOut - 1 + lane, r0 = y0 + i * c.block_rows;
-        if (lane >= 1 && lane <= kStripOut && gx < c.nx)
-          for (int r = r0; r < min(r0 + c.block_rows, y1); ++r) {
-            const size_t gi = (size_t)r * c.pitch + gx;
-            hdst[gi] = 0;
-            qxdst[gi] = 0.f;
-            qydst[gi] = 0.f;
-          }
-        if (lane == 0) next[own + i] = 0;
+        for (int t = 0; t < kFvChunkBlocks; ++t) {
+          if (t >= shared) break;
+          const int q = chunk_of(t), qj = q / c.tiles_x;
+          const int fi = lane / 3 - 1, fs = q - qj * c.tiles_x - 1 + lane % 3;
+          const bool in = fs >= 0 && fs < c.tiles_x &&
+                          (fi < 0                ? qj > 0
+                           : fi < c.chunk_blocks ? qj * c.chunk_rows + fi * c.block_rows < c.ny
+                                                 : fi == c.chunk_blocks && qj + 1 < c.row_chunks);
+          const int f = in ? __ldcg(wet + fs * column + qj * c.chunk_blocks + fi) : 0;
+          unsigned m = __ballot_sync(0xffffffffu, f != 0);
+          if (__all_sync(0xffffffffu, f || !in)) m |= 0x80000000u;
+          if (lane == 0) near[warp][t] = m;
+        }
+        const unsigned stale =
+            __ballot_sync(0xffffffffu, lane < blocks && __ldcg(next + own + lane) != 0);
+        __syncwarp();
+        for (int i = 0; i < blocks; ++i) {
+          // dry, and the other buffer is not
+          if ((near[warp][0] >> (3 * i)) & 0x1ffu || !((stale >> i) & 1u)) continue;
+          const int gx = strip * kStripOut - 1 + lane, r0 = y0 + i * c.block_rows;
+          if (lane >= 1 && lane <= kStripOut && gx < c.nx)
+            for (int r = r0; r < min(r0 + c.block_rows, y1); ++r) {
+              const size_t gi = (size_t)r * c.pitch + gx;
+              hdst[gi] = 0;
+              qxdst[gi] = 0.f;
+              qydst[gi] = 0.f;
+            }
+          if (lane == 0) next[own + i] = 0;
+        }
       }
       for (int t = 0; t < shared; ++t) {
         const unsigned m = near[warp][t];
@@ -998,7 +1022,8 @@ __global__ void __launch_bounds__(kThreads, 4)
         // the grid is; else single blocks, shared out
         const bool runs = dense || (m >> 31);
         if (runs && t > 0) continue;
-        const int q = chunk_of(t), qj = q / c.tiles_x, qs = q - qj * c.tiles_x;
+        const int q = chunk_of(t), qj = t == 0 ? j : q / c.tiles_x;
+        const int qs = q - qj * c.tiles_x;
         const int q0 = qj * c.chunk_rows, q1 = min(q0 + c.chunk_rows, c.ny);
         const int end = runs ? blocks : t + 1;
         for (int i = runs ? 0 : t; i < end;) {
@@ -1020,31 +1045,28 @@ __global__ void __launch_bounds__(kThreads, 4)
     }
 #pragma unroll
     for (int q = 0; q < kFvDiag; ++q) sums[q][threadIdx.x] += (double)fa[q];
-    double wave = (double)fwave;
-    wave = warp_max(wave);
-    if (lane == 0) {
-      wred[warp] = wave;
-      nred[warp] = wet_blocks;
-    }
+    const unsigned wave = __reduce_max_sync(0xffffffffu, __float_as_uint(fwave));
+    if (lane == 0) wred[warp] = make_uint2(wave, (unsigned)wet_blocks);
     // the CTA barrier orders every thread's field writes before thread 0's
     // device-scope fence and arrival (the grid-barrier pattern: one fence)
     __syncthreads();
     if (threadIdx.x == 0) {
-      double m = 0.0;
+      unsigned m = 0, n = 0;
 #pragma unroll
-      for (int w = 0; w < kThreads / 32; ++w) m = fmax(m, wred[w]);
-      atomicMax(&ctl->wave3[k % 3], (unsigned long long)__double_as_longlong(m));
-      int n = 0;
-#pragma unroll
-      for (int w = 0; w < kThreads / 32; ++w) n += nred[w];
-      if (n) atomicAdd(&ctl->wetn[k % 3], n);
+      for (int w = 0; w < kThreads / 32; ++w) {
+        m = max(m, wred[w].x);
+        n += wred[w].y;
+      }
+      atomicMax(&ctl->wave3[k % 3],
+                (unsigned long long)__double_as_longlong((double)__uint_as_float(m)));
       __threadfence();
-      const unsigned prev = atomicAdd(&ctl->arrive, 1u);
+      const unsigned long long prev =
+          atomicAdd(&ctl->arrive_wet, ((unsigned long long)n << 32) + 1ull);
       bool failed = false;
-      if (prev == gridDim.x - 1) {
-        ctl->arrive = 0;
+      if ((unsigned)prev == gridDim.x - 1) {
+        ctl->arrive_wet = 0ull;
         ctl->wave3[(k + 1) % 3] = 0ull;  // read by every CTA two barriers ago
-        ctl->wetn[(k + 1) % 3] = 0;
+        ctl->wetn[k % 3] = (int)((unsigned)(prev >> 32) + n);
         __threadfence();
         atomicAdd(&ctl->gen, 1u);  // release
       } else {
@@ -1069,7 +1091,7 @@ __global__ void __launch_bounds__(kThreads, 4)
       } else {
         const double w = __longlong_as_double((long long)__ldcg(&ctl->wave3[k % 3]));
         L.wave = w;
-        L.dense = 2 * (long long)__ldcg(&ctl->wetn[k % 3]) >= (long long)c.tiles_x * column;
+        L.dense = fv_dense(__ldcg(&ctl->wetn[k % 3]), every);
         if (!(L.remaining > 1.0e-14)) {
           L.done = 1;
         } else if (L.substeps >= c.max_substeps) {

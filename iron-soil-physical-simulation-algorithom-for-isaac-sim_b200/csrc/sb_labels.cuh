@@ -99,6 +99,11 @@ __device__ __forceinline__ double free_surface_diff(const typename FvTypes<FX>::
 struct YieldF {
   float sx[2], sy[2];
   float Q, depth, rg, coh, ts, tp, dts, dry;
+  // A gradient below this is stable against both angles whatever the layer:
+  // 1e-5 under the smaller tangent, where the margins' float32 rounding stays
+  // below 1e-6 of the friction term; negative (never) for parameters of other
+  // signs.
+  float calm;
 };
 
 __device__ __forceinline__ YieldF yield_constants(const LabelConst& c) {
@@ -115,6 +120,9 @@ __device__ __forceinline__ YieldF yield_constants(const LabelConst& c) {
   y.tp = (float)c.tan_stop;
   y.dts = (float)(c.tan_start - c.tan_stop);
   y.dry = (float)c.dry;
+  y.calm = y.coh >= 0.f && y.rg > 0.f && y.ts > 0.f && y.tp > 0.f && y.depth > 0.f
+               ? fminf(y.ts, y.tp) * (1.f - 1.0e-5f)
+               : -1.f;
   return y;
 }
 
@@ -126,7 +134,8 @@ __device__ __forceinline__ YieldF yield_constants(const LabelConst& c) {
 // the exact value <= 2e-7 rad.
 __device__ __forceinline__ float atan_as4449(float x) {
   const bool inv = x > 1.0f;
-  const float t = inv ? 1.0f / x : x;
+  float t = x;
+  if (inv) t = 1.0f / x;
   const float t2 = t * t;
   float p = 0.0028662257f;
   p = -0.0161657367f + t2 * p;
@@ -215,6 +224,7 @@ __global__ void __launch_bounds__(kLabelInitThreads, 3)
   const typename FvTypes<FX>::R* qx = P ? qx1 : qx0;
   const typename FvTypes<FX>::R* qy = P ? qy1 : qy0;
   const YieldF yf = yield_constants(c);
+  int any = 0;
   for (int li = threadIdx.x; li < kLabelTile * kLabelTile; li += kLabelInitThreads) {
     const int ly = li / kLabelTile, lx = li % kLabelTile;
     const int r = gy0 + ly, col = gx0 + lx;
@@ -234,22 +244,29 @@ __global__ void __launch_bounds__(kLabelInitThreads, 3)
                               ((long long)b[(size_t)r * c.pitch + cl] + h[(size_t)r * c.pitch + cl]);
         const long long dyq = ((long long)b[(size_t)ru * c.pitch + col] + h[(size_t)ru * c.pitch + col]) -
                               ((long long)b[(size_t)rd * c.pitch + col] + h[(size_t)rd * c.pitch + col]);
-        const float gx = (float)dxq * (inx ? yf.sx[0] : yf.sx[1]);
-        const float gy = (float)dyq * (iny ? yf.sy[0] : yf.sy[1]);
+        // (the 32-bit conversion rounds alike and is four times as fast)
+        const float gx = ((int)dxq == dxq ? (float)(int)dxq : (float)dxq) *
+                         (inx ? yf.sx[0] : yf.sx[1]);
+        const float gy = ((int)dyq == dyq ? (float)(int)dyq : (float)dyq) *
+                         (iny ? yf.sy[0] : yf.sy[1]);
         const float mag = sqrtf(gx * gx + gy * gy);
         const long long dq = (long long)b[gi] - (long long)z[gi];
-        const float layer = fminf((float)(dq > 0 ? dq : 0) * yf.Q, yf.depth);
         mob = (double)h[gi] * c.Q;
-        const float norm = sqrtf(1.0f + mag * mag);
-        const float drive = yf.rg * layer * mag / norm;
-        const float normal = yf.rg * layer / norm;
-        const float start_margin = drive - (yf.coh + normal * yf.ts);
-        const float stop_margin = drive - (yf.coh + normal * yf.tp);
-        const float sev = fminf(fmaxf(stop_margin / fmaxf(normal * yf.dts, 1.0e-12f), 0.f), 1.f);
         slope_out[flat] = atan_as4449(mag);
+        float sev = 0.f;
+        settled = true;
+        if (!(mag < yf.calm)) {  // nearly all cells are calm: no roots, no divisions
+          const float layer = fminf((float)(dq > 0 ? dq : 0) * yf.Q, yf.depth);
+          const float norm = sqrtf(1.0f + mag * mag);
+          const float drive = yf.rg * layer * mag / norm;
+          const float normal = yf.rg * layer / norm;
+          const float start_margin = drive - (yf.coh + normal * yf.ts);
+          const float stop_margin = drive - (yf.coh + normal * yf.tp);
+          sev = fminf(fmaxf(stop_margin / fmaxf(normal * yf.dts, 1.0e-12f), 0.f), 1.f);
+          u = (layer > yf.dry && start_margin > 0.f) ? 1 : 0;
+          settled = stop_margin <= 0.f;
+        }
         severity_out[flat] = sev;
-        u = (layer > yf.dry && start_margin > 0.f) ? 1 : 0;
-        settled = stop_margin <= 0.f;
       } else {
         const double denx = inx ? 2.0 * c.dx : c.dx;
         const double deny = iny ? 2.0 * c.dy : c.dy;
@@ -296,7 +313,9 @@ __global__ void __launch_bounds__(kLabelInitThreads, 3)
       }
     }
     lab[li] = u ? li : -1;
+    any |= u;
   }
+  if (!__syncthreads_or(any)) return;  // no unstable cell in the tile
   local_ccl(lab, c.connectivity, gy0, gx0, c.nx, parent);
 }
 

@@ -161,6 +161,7 @@ struct sb_ctx {
   int fv_strips = 0;
   int fv_stream_blocks = 0;
   int ledger_blocks = 0;
+  int ledger_grid = 0;  // blocks of the ledger kernel, at most ledger_blocks
   MobileGraph mobile;
   cudaEvent_t ev_loop[2] = {nullptr, nullptr};  // around the substep WHILE node
   cudaEvent_t ev_path[2] = {nullptr, nullptr};  // first and last node of the step graph
@@ -514,7 +515,7 @@ int build_mobile_graph(sb_ctx* ctx, const FvConst& c, double static_limit) {
     int pro_handle = (FX && ctx->fv_stream && ctx->fv_persistent) ? 0 : use_handle;
     ledger_args<FX>(ctx, cc, &datum, &limit, &mode0, &handle, &pro_handle, args);
     int rc = add_kernel(ctx, g, &n_pro, &n_begin, 1, (void*)ledger_kernel<FX>,
-                        dim3(ctx->ledger_blocks), 0, args.data());
+                        dim3(ctx->ledger_grid), 0, args.data());
     if (rc) return rc;
   }
   cudaGraphNode_t n_ev0, n_ev1;
@@ -529,7 +530,7 @@ int build_mobile_graph(sb_ctx* ctx, const FvConst& c, double static_limit) {
     ledger_args<FX>(ctx, cc, &datum, &limit, &mode1, &handle, &no_handle, args);
     SB_CUDA(ctx, cudaGraphAddEventRecordNode(&n_ev1, g, &n_loop, 1, ctx->ev_loop[1]));
     int rc = add_kernel(ctx, g, &n_after, &n_ev1, 1, (void*)ledger_kernel<FX>,
-                        dim3(ctx->ledger_blocks), 0, args.data());
+                        dim3(ctx->ledger_grid), 0, args.data());
     if (rc) return rc;
   }
   {
@@ -615,7 +616,7 @@ static int mobile_step_host_loop(sb_ctx* ctx, const FvConst& c, double static_li
   }
   std::vector<void*> args;
   ledger_args<FX>(ctx, cc, &datum, &limit, &mode0, &handle, &no_handle, args);
-  SB_CUDA(ctx, cudaLaunchKernel((void*)ledger_kernel<FX>, dim3(ctx->ledger_blocks), dim3(kThreads),
+  SB_CUDA(ctx, cudaLaunchKernel((void*)ledger_kernel<FX>, dim3(ctx->ledger_grid), dim3(kThreads),
                                 args.data(), 0, ctx->stream));
   SB_CUDA(ctx, cudaEventRecord(ctx->ev_loop[0], ctx->stream));
   if (FX && ctx->fv_stream && ctx->fv_persistent) {
@@ -641,7 +642,7 @@ static int mobile_step_host_loop(sb_ctx* ctx, const FvConst& c, double static_li
   SB_CUDA(ctx, cudaEventRecord(ctx->ev_loop[1], ctx->stream));
   std::vector<void*> a2;
   ledger_args<FX>(ctx, cc, &datum, &limit, &mode1, &handle, &no_handle, a2);
-  SB_CUDA(ctx, cudaLaunchKernel((void*)ledger_kernel<FX>, dim3(ctx->ledger_blocks), dim3(kThreads),
+  SB_CUDA(ctx, cudaLaunchKernel((void*)ledger_kernel<FX>, dim3(ctx->ledger_grid), dim3(kThreads),
                                 a2.data(), 0, ctx->stream));
   return SB_OK;
 }
@@ -794,6 +795,13 @@ int sb_ctx_create(const sb_grid_desc* desc, sb_ctx** out) {
   // grid-stride reductions: three CTAs per SM (the ledger kernel's register
   // bound) keep the final fold short
   ctx->ledger_blocks = std::min(grid_for((long long)d.ny * d.nx), 3 * 148);
+  ctx->ledger_grid = ctx->ledger_blocks;
+  if (fx(ctx)) {
+    const long long items = (long long)d.ny * ((d.nx + kLedgerCols - 1) / kLedgerCols);
+    ctx->ledger_grid =
+        (int)std::min({(items + kThreads / 32 - 1) / (kThreads / 32),
+                       (long long)kLedgerCtasFx * 148, (long long)ctx->ledger_blocks});
+  }
   const size_t np = (size_t)std::max({tiles, ctx->ledger_blocks, ctx->fv_stream_blocks}) *
                     (kFvPartial > L_NP ? kFvPartial : L_NP);
   dev.add(&ctx->partials, np * sizeof(double));
@@ -1222,7 +1230,7 @@ int sb_mobile_ledger_of(sb_ctx* ctx, const sb_mobile_params* params, sb_mobile_l
   else
     ledger_args<false>(ctx, c, &datum, &limit, &mode, &handle, &use_handle, args);
   void* fn = fx(ctx) ? (void*)ledger_kernel<true> : (void*)ledger_kernel<false>;
-  SB_CUDA(ctx, cudaLaunchKernel(fn, dim3(ctx->ledger_blocks), dim3(kThreads), args.data(), 0,
+  SB_CUDA(ctx, cudaLaunchKernel(fn, dim3(ctx->ledger_grid), dim3(kThreads), args.data(), 0,
                                 ctx->stream));
   ctx->launches++;
   SB_CUDA(ctx, cudaMemcpyAsync(ctx->io_host, ctx->io, sizeof(StepIO), cudaMemcpyDeviceToHost,
@@ -2255,7 +2263,7 @@ int build_path_graph(sb_ctx* ctx, const sb_path_params* p) {
     int pro_h = (FX && ctx->fv_stream && ctx->fv_persistent) ? 0 : use_h;
     std::vector<void*> args;
     ledger_args<FX>(ctx, fc, &dat, &static_limit, &mode0, &h_mob, &pro_h, args);
-    if ((rc = add_kernel(ctx, g, &node, &prev, 1, (void*)ledger_kernel<FX>, dim3(ctx->ledger_blocks),
+    if ((rc = add_kernel(ctx, g, &node, &prev, 1, (void*)ledger_kernel<FX>, dim3(ctx->ledger_grid),
                          0, args.data())))
       return rc;
     prev = node;
@@ -2290,7 +2298,7 @@ int build_path_graph(sb_ctx* ctx, const sb_path_params* p) {
     std::vector<void*> args;
     ledger_args<FX>(ctx, fc, &dat, &static_limit, &mode1, &h_mob, &no_h, args);
     if ((rc = add_kernel(ctx, g, &n_after, &prev, 1, (void*)ledger_kernel<FX>,
-                         dim3(ctx->ledger_blocks), 0, args.data())))
+                         dim3(ctx->ledger_grid), 0, args.data())))
       return rc;
     if ((rc = mark())) return rc;
   }
