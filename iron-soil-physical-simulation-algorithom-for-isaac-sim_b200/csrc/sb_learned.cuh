@@ -48,10 +48,11 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
-// kind::f16 instruction descriptor: D f32, A/B bf16, both K-major.
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(m >> 4) << 24);
+// kind::f16 instruction descriptor: D f32, A/B bf16, both K-major or both
+// MN-major.
+__host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n, bool mn_major = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major ? 3u << 15 : 0u) |
+         ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
@@ -121,10 +122,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ uint32_t core_off(int r, int k, int kdim) {
-  return (uint32_t)(((r >> 3) * (kdim >> 3) + (k >> 3)) * 128 + (r & 7) * 16 + (k & 7) * 2);
 }
 
 struct ConvArgs {
@@ -534,149 +531,209 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_rot_kernel(const ConvArg
 struct WgradArgs {
   const __nv_bfloat16* in;    // layer input [batch][h][w][cin]
   const __nv_bfloat16* grad;  // gradient at the layer output [batch][h][w][cout]
-  float* partial;             // per CTA: [3 dy][128 (dx, ci)][cout]
+  float* partial;             // per CTA: [3 dy][3 dx][cin][cout]
   int batch, h, w;
-  int rows_per_cta;
+  int rows;    // output rows of a band
+  int tiles;   // bands side by side (128 pixels each)
+  int chunks;  // bands over the height
+  int bands;   // of a CTA: 1 or kWgradBands
   int* status;
 };
 
+constexpr int kWgradBands = 2;
+constexpr int kWgradSlots = 4;
+
 template <int CIN, int COUT>
 struct WgradSmem {
-  static constexpr int T_BYTES = 128 * 128 * 2;       // A: (dx, ci) rows x 128 pixels
-  static constexpr int G_BYTES = COUT * 128 * 2;      // B: co rows x 128 pixels
-  static constexpr int BYTES = T_BYTES + 3 * G_BYTES + 64;
-  static constexpr uint32_t TMEM_COLS = 3 * COUT <= 64 ? 64 : 128;
+  static constexpr uint32_t ROW = 4 * kRowLbo;  // input row: room for 32 channels
+  static constexpr uint32_t G_ROW = (COUT / 8) * kRowLbo;
+  static constexpr uint32_t BAND = kWgradSlots * ROW + 2 * G_ROW;
+  static constexpr uint32_t FOLD = 9 * CIN * (COUT + 1) * 4;  // in the place of the bands
+  static constexpr uint32_t USED = kWgradBands * BAND > FOLD ? kWgradBands * BAND : FOLD;
+  // above half an SM's shared memory where a CTA takes all TMEM columns
+  static constexpr uint32_t BYTES = (COUT == 32 && USED < 118 * 1024 ? 118 * 1024 : USED) + 64;
+  static constexpr uint32_t TMEM_COLS = COUT == 32 ? 512 : 256;  // 4 phases x 3 dx x COUT
 };
 
+// Starts the copy of pixels [x, x + n) of an image row of C channels into a
+// staged row: 16-byte pieces, neighbouring threads on neighbouring addresses;
+// zeros outside the image.
+template <int C>
+__device__ __forceinline__ void wgrad_row_async(const __nv_bfloat16* __restrict__ image, int h,
+                                                int w, int r, int x, int n, uint32_t dst) {
+  const bool row = r >= 0 && r < h;
+  const __nv_bfloat16* src = image + (size_t)(row ? r : 0) * w * C;
+  for (int i = threadIdx.x; i < n * (C / 8); i += kConvThreads) {
+    const int p = i / (C / 8), c8 = i % (C / 8);
+    const bool ok = row && x + p >= 0 && x + p < w;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + c8 * kRowLbo + p * 16),
+                 "l"(src + (ok ? (size_t)(x + p) * C : 0) + c8 * 8), "r"(ok ? 16u : 0u)
+                 : "memory");
+  }
+}
+
+// dW[dy][dx][ci][co] = sum over pixels of in[y + dy - 1][x + dx - 1][ci] g[y][x][co].
+//
+// Both operands are contracted over pixels, so both are MN-major in the staged rows
+// as they lie in memory (16 bytes = 8 channels of a pixel; core matrices of 8 pixels,
+// 128 B apart along K; channel groups kRowLbo apart along M and N): nothing is
+// transposed, and a dx is the same rows dx * 16 bytes on.  The four slots of the row
+// ring are M = 4 x 32 channels: at output row y three of them are dy = 0, 1, 2 and the
+// fourth, which takes row y + 2 meanwhile, gives products that are never read.  Which
+// slot is which dy depends on y mod 4, so each of the four phases has its own three
+// (dx) accumulators of COUT columns.  A step of a CTA is one output row of each of its
+// bands; the next rows are in flight during its MMAs.
+//
+// Bound by the rows' way through shared memory (67 MB for 32 images of 128 x 128 x 32,
+// mostly from L2).  Transposing each row with 2-byte stores and waiting for its MMAs
+// took 147 to 186 us there, this takes 57 to 61.
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_tc_kernel(const WgradArgs a) {
   using S = WgradSmem<CIN, COUT>;
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* tbuf = smem;
-  unsigned char* gring = smem + S::T_BYTES;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(gring + 3 * S::G_BYTES);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int x0 = blockIdx.x * 128;
-  const int y0 = blockIdx.y * a.rows_per_cta;
-  const int y1 = min(y0 + a.rows_per_cta, a.h);
-  const int b = blockIdx.z;
-  const size_t cta = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S::BYTES - 64);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t base = smem_u32(smem);
 
-  // zero A (the (dx, ci) rows beyond 3*CIN stay zero)
-  for (int i = tid; i < S::T_BYTES / 16; i += kConvThreads)
-    reinterpret_cast<uint4*>(tbuf)[i] = make_uint4(0, 0, 0, 0);
-  if (tid == 0) mbar_init(bar, 1);
-  if (warp == 0) tmem_alloc(tslot, S::TMEM_COLS);
-
-  // gradient row r -> ring slot (B operand: element (co, pixel k))
-  auto load_grad = [&](int r) {
-    unsigned char* dst = gring + ((r + 3) % 3) * S::G_BYTES;
-    const int k = tid, x = x0 + k;
-    const bool okp = r >= 0 && r < a.h && x < a.w;
-    const __nv_bfloat16* src = a.grad + (((size_t)b * a.h + (okp ? r : 0)) * a.w + (okp ? x : 0)) * COUT;
+  int y0[kWgradBands], y1[kWgradBands], x0[kWgradBands], npx[kWgradBands];
+  const __nv_bfloat16 *in[kWgradBands], *grad[kWgradBands];
+  int steps = 0;
 #pragma unroll
-    for (int co = 0; co < COUT; ++co) {
-      const __nv_bfloat16 v = okp ? src[co] : __float2bfloat16_rn(0.f);
-      *reinterpret_cast<__nv_bfloat16*>(dst + core_off(co, k, 128)) = v;
-    }
+  for (int n = 0; n < kWgradBands; ++n) {
+    const int items = a.tiles * a.chunks * a.batch;
+    const int it = blockIdx.x * a.bands + n;
+    const bool has = n < a.bands && it < items;
+    const int q = has ? it / a.tiles : 0, img = q / a.chunks;
+    x0[n] = has ? (it - q * a.tiles) * 128 : 0;
+    y0[n] = has ? (q - img * a.chunks) * a.rows : 0;
+    y1[n] = has ? min(y0[n] + a.rows, a.h) : 0;
+    npx[n] = (min(a.w - x0[n], 128) + 15) / 16 * 16;  // K of its MMAs
+    in[n] = a.in + (size_t)img * a.h * a.w * CIN;
+    grad[n] = a.grad + (size_t)img * a.h * a.w * COUT;
+    steps = max(steps, y1[n] - y0[n]);
+  }
+  auto slot = [&](int n, int r) { return base + n * S::BAND + ((r + 4) & 3) * S::ROW; };
+  auto gslot = [&](int n, int y) {
+    return base + n * S::BAND + kWgradSlots * S::ROW + (y & 1) * S::G_ROW;
   };
-  load_grad(y0 - 1);
-  load_grad(y0);
-  fence_async_smem();
+  auto load_in = [&](int n, int r) {
+    if (y0[n] < y1[n] && r <= y1[n])
+      wgrad_row_async<CIN>(in[n], a.h, a.w, r, x0[n] - 1, npx[n] + 2, slot(n, r));
+  };
+  auto load_grad = [&](int n, int y) {
+    if (y < y1[n]) wgrad_row_async<COUT>(grad[n], a.h, a.w, y, x0[n], npx[n], gslot(n, y));
+  };
+#pragma unroll
+  for (int n = 0; n < kWgradBands; ++n) {
+    load_in(n, y0[n] - 1);
+    load_in(n, y0[n]);
+    load_in(n, y0[n] + 1);
+    load_grad(n, y0[n]);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  if (tid == 0) {
+    mbar_init(bar, 1);
+    mbar_init(bar + 1, 1);
+  }
+  if (warp == 0) tmem_alloc(tslot, S::TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tslot;
-  const uint32_t idesc = umma_idesc_bf16(128, COUT);
-  const uint32_t t_base = smem_u32(tbuf), g_base = smem_u32(gring);
-  const uint32_t lbo = 128;
-  unsigned phase = 0;
+  const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 1
+  for (int k = 0; k < 12; ++k) tmem_zero<COUT>(lane_addr + (uint32_t)(k * COUT));
+  tc_fence_before();
+  const uint32_t idesc = umma_idesc_bf16(128, COUT, true);
   bool ok = true;
-  int started[3] = {0, 0, 0};
-
-  // input rows r contribute to output rows y = r - dy + 1 in [y0, y1)
-  for (int r = y0 - 1; r <= y1; ++r) {
-    if (r + 1 <= y1) load_grad(r + 1);
-    // A: element ((dx, ci), k) = input[r][x0 + k + dx - 1][ci]
-    if (r >= 0 && r < a.h) {
-      for (int j = tid; j < 130; j += kConvThreads) {
-        const int x = x0 + j - 1;
-        const bool okp = x >= 0 && x < a.w;
-        const __nv_bfloat16* src = a.in + (((size_t)b * a.h + r) * a.w + (okp ? x : 0)) * CIN;
-        for (int ci = 0; ci < CIN; ++ci) {
-          const __nv_bfloat16 v = okp ? src[ci] : __float2bfloat16_rn(0.f);
-#pragma unroll
-          for (int dx = 0; dx < 3; ++dx) {
-            const int k = j - dx;
-            if (k >= 0 && k < 128)
-              *reinterpret_cast<__nv_bfloat16*>(tbuf + core_off(dx * CIN + ci, k, 128)) = v;
-          }
-        }
-      }
-    } else {
-      for (int i = tid; i < (3 * CIN) * 128 / 8; i += kConvThreads) {
-        const int row = i / 16, kb = i % 16;
-        *reinterpret_cast<uint4*>(tbuf + core_off(row, kb * 8, 128)) = make_uint4(0, 0, 0, 0);
-      }
-    }
+  for (int i = 0; i < steps; ++i) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     fence_async_smem();
-    __syncthreads();
-    bool issued = false;
+    __syncthreads();  // rows y - 1 .. y + 1 and the gradient row are staged
     if (tid == 0) {
       tc_fence_after();
-      for (int dy = 0; dy < 3; ++dy) {
-        const int y = r - dy + 1;
-        if (y < y0 || y >= y1) continue;
-        const uint32_t g_row = g_base + ((y + 3) % 3) * S::G_BYTES;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16(tmem + dy * COUT, umma_desc(t_base + kk * 256, lbo, 16 * 128),
-                    umma_desc(g_row + kk * 256, lbo, 16 * 128), idesc, started[dy] | (kk > 0));
-        started[dy] = 1;
-        issued = true;
+      for (int n = 0; n < kWgradBands; ++n) {
+        const int y = y0[n] + i;
+        if (y >= y1[n]) continue;
+        const uint64_t adesc = umma_desc(slot(n, 0), 128, kRowLbo);
+        const uint64_t bdesc = umma_desc(gslot(n, y), 128, kRowLbo);
+        const uint32_t d = tmem + (uint32_t)((y & 3) * 3 * COUT);
+        for (int kk = 0; kk < npx[n] / 16; ++kk)
+#pragma unroll
+          for (int dx = 0; dx < 3; ++dx)
+            umma_bf16(d + dx * COUT, adesc + (uint64_t)(kk * 16 + dx),
+                      bdesc + (uint64_t)(kk * 16), idesc, 1);
       }
-      if (issued) umma_commit(bar);
+      umma_commit(bar + (i & 1));
     }
-    issued = __syncthreads_or(issued ? 1 : 0);
-    if (issued) {
-      ok = mbar_wait(bar, phase) && ok;
-      phase ^= 1;
+    // the previous step's MMAs have read the slots that the next rows take
+    if (i > 0) ok = mbar_wait(bar + ((i - 1) & 1), ((i - 1) >> 1) & 1) && ok;
+    if (i + 1 < steps) {
+#pragma unroll
+      for (int n = 0; n < kWgradBands; ++n) {
+        load_in(n, y0[n] + i + 2);
+        load_grad(n, y0[n] + i + 1);
+      }
     }
-    tc_fence_after();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  if (steps > 0) ok = mbar_wait(bar + ((steps - 1) & 1), ((steps - 1) >> 1) & 1) && ok;
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  tc_fence_after();
+  __syncthreads();  // every MMA has completed: the rows' place takes the sums
+  // warp = slot, lane = ci.  Slot s holds dy at phase p = s + 1 - dy (mod 4).  The
+  // warps take the taps in turn, four groups of them in four rounds, so each tap's
+  // four shares are added in a fixed order.
+  float* fold = reinterpret_cast<float*>(smem);
+#pragma unroll 1
+  for (int round = 0; round < 4; ++round) {
+#pragma unroll 1
+    for (int tap = (warp + round) & 3; tap < 9; tap += 4) {
+      const int dy = tap / 3, dx = tap - dy * 3;
+      float v[COUT];
+      const uint32_t col = (uint32_t)((((warp + 5 - dy) & 3) * 3 + dx) * COUT);
+      if constexpr (COUT == 32)
+        tmem_ld32(lane_addr + col, v);
+      else
+        tmem_ld16(lane_addr + col, v);
+      if (lane < CIN) {
+        float* f = fold + (tap * CIN + lane) * (COUT + 1);
+#pragma unroll
+        for (int co = 0; co < COUT; ++co) f[co] = round == 0 ? v[co] : f[co] + v[co];
+      }
+    }
     __syncthreads();
   }
-  // epilogue: lane m = (dx, ci), columns (dy, co)
-  tc_fence_after();
-  const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-  float* out = a.partial + cta * (size_t)(3 * 128 * COUT);
-  for (int dy = 0; dy < 3; ++dy) {
-#pragma unroll
-    for (int c = 0; c < COUT; c += 16) {
-      float v[16];
-      tmem_ld16(lane_addr + dy * COUT + c, v);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) out[((size_t)dy * 128 + tid) * COUT + c + j] = y0 < y1 ? v[j] : 0.f;
-    }
-  }
+  float* out = a.partial + (size_t)blockIdx.x * (9 * CIN * COUT);
+  for (int i = tid; i < 9 * CIN * COUT; i += kConvThreads)
+    out[i] = fold[i / COUT * (COUT + 1) + i % COUT];
   if (!ok && tid == 0 && a.status) atomicExch(a.status, 1);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_free(tmem, S::TMEM_COLS);
 }
 
-// dW[dy][dx][ci][co] = sum over CTAs (fixed order) of partial[cta][dy][dx*cin+ci][co].
-__global__ void wgrad_reduce_kernel(const float* __restrict__ partial, int nctas, int cin, int cout,
-                                    float* __restrict__ dw) {
-  const int n = 9 * cin * cout;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int co = i % cout;
-    const int ci = (i / cout) % cin;
-    const int dx = (i / (cout * cin)) % 3;
-    const int dy = i / (3 * cout * cin);
-    const size_t off = ((size_t)dy * 128 + dx * cin + ci) * cout + co;
-    double s = 0.0;
-    for (int c = 0; c < nctas; ++c) s += (double)partial[(size_t)c * 3 * 128 * cout + off];
+// dw[i] = sum over CTAs of partial[cta][i], in FP64 and a fixed order: 32 outputs per
+// block, eight threads each (one thread per output read 256 CTAs one after another:
+// 25 us).
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ partial,
+                                                           int nctas, int n,
+                                                           float* __restrict__ dw) {
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  double s = 0.0;
+  if (i < n) {
+#pragma unroll 4
+    for (int c = slice; c < nctas; c += 8) s += (double)partial[(size_t)c * n + i];
+  }
+  part[slice][lane] = s;
+  __syncthreads();
+  if (slice == 0 && i < n) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += part[k][lane];
     dw[i] = (float)s;
   }
 }
@@ -735,20 +792,10 @@ __global__ void learned_features_kernel(const LearnedGeom g, const HT* __restric
   }
 }
 
-// Proposed transfer on edge k of cell c, in metres: flux * tan_crit * dx,
-// limited to half the height difference across that edge (the proposal never
-// reverses a difference on its own).  Edges leaving the grid carry nothing.
-__device__ __forceinline__ double learned_transfer(const LearnedGeom& g, double flux, double hc,
-                                                   double hn) {
-  const double t = flux * g.tan_crit * g.dx;
-  const double lim = 0.5 * fabs(hc - hn);
-  return fmin(fmax(t, -lim), lim);
-}
-
 // Fixed point: transfers in whole quanta per edge (int32 [pixel][4]), rounded
 // toward zero, then gathered -- every quantum leaves one cell and enters one
 // neighbour.  Q is a power of two, so scaling by it commutes with every
-// rounding, and truncation with learned_transfer's clamp to half the (whole)
+// rounding, and truncation with the clamp to half the (whole)
 // height difference: trunc(clamp(t, lim) / Q) = clamp(trunc(t / Q), |dq| / 2).
 // Four dependent double operations instead of fifteen.
 __device__ __forceinline__ int learned_quanta(float flux, int hc, int hn, double tan_crit,

@@ -50,8 +50,9 @@ cudaError_t launch_wgrad(const WgradArgs& a, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  dim3 grid((a.w + 127) / 128, (a.h + a.rows_per_cta - 1) / a.rows_per_cta, a.batch);
-  conv3x3_wgrad_tc_kernel<CIN, COUT><<<grid, kConvThreads, S::BYTES, st>>>(a);
+  const int items = a.tiles * a.chunks * a.batch;
+  conv3x3_wgrad_tc_kernel<CIN, COUT>
+      <<<(items + a.bands - 1) / a.bands, kConvThreads, S::BYTES, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -180,8 +181,11 @@ int sb_learned_wgrad(const void* in, const void* grad, float* partial, size_t pa
   const size_t nctas = (size_t)((w + 127) / 128) * ((h + rows_per_cta - 1) / rows_per_cta) * batch;
   if (partial_floats < nctas * 3 * 128 * (size_t)cout)
     return lfail(SB_ERR_CAPACITY, "[soilb200] wgrad: partial buffer too small");
+  if (batch > 65535 || (h + rows_per_cta - 1) / rows_per_cta > 65535)
+    return lcuda(cudaErrorInvalidConfiguration);
   WgradArgs a{(const __nv_bfloat16*)in, (const __nv_bfloat16*)grad, partial, batch, h, w,
-              rows_per_cta, d_status};
+              rows_per_cta, (w + 127) / 128, (h + rows_per_cta - 1) / rows_per_cta,
+              nctas > 148 ? kWgradBands : 1, d_status};
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e;
   if (cin == 16 && cout == 32) e = launch_wgrad<16, 32>(a, st);
@@ -189,7 +193,8 @@ int sb_learned_wgrad(const void* in, const void* grad, float* partial, size_t pa
   else if (cin == 32 && cout == 16) e = launch_wgrad<32, 16>(a, st);
   else e = launch_wgrad<16, 16>(a, st);
   if (e != cudaSuccess) return lcuda(e);
-  wgrad_reduce_kernel<<<(9 * cin * cout + 255) / 256, 256, 0, st>>>(partial, (int)nctas, cin, cout, dw);
+  const int n = 9 * cin * cout, ctas = ((int)nctas + a.bands - 1) / a.bands;
+  wgrad_reduce_kernel<<<(n + 31) / 32, 256, 0, st>>>(partial, ctas, n, dw);
   return lcuda(cudaGetLastError());
 }
 

@@ -1,0 +1,33 @@
+"""The weight-gradient kernel at the edges of its bands: widths around a
+16-pixel MMA step and a 128-pixel band, heights around the rows of a band, one
+and two bands per CTA (more than 148 bands), every channel pair, against the
+oracle.  Bound: products of BF16 values are exact in FP32, so an output is off
+by at most the roundings of a sum of n terms, n 2^-24 of the magnitudes' sum."""
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from oracle import learned as L  # noqa: E402
+from soilb200 import learned as ln  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def _bf16(rng, *shape):
+    return torch.as_tensor(rng.normal(size=shape)).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 16), (32, 32)])
+@pytest.mark.parametrize("b,h,w,rows", [(1, 1, 1, 16), (1, 3, 15, 2), (2, 5, 16, 1), (1, 9, 17, 4),
+                                        (2, 17, 127, 16), (1, 18, 128, 5), (1, 6, 129, 3),
+                                        (3, 34, 260, 16), (40, 16, 24, 4), (149, 4, 8, 16)])
+def test_wgrad_band_edges(b, h, w, rows, cin, cout):
+    rng = np.random.default_rng(b * 1000 + h * 10 + w)
+    x, g = _bf16(rng, b, h, w, cin), _bf16(rng, b, h, w, cout)
+    got = ln.wgrad(x.cuda(), g.cuda(), cin, cout, rows=rows).cpu().numpy().astype(np.float64)
+    xd, gd = x.double().numpy(), g.double().numpy()
+    want = L.conv3x3_wgrad(xd, gd)
+    size = L.conv3x3_wgrad(np.abs(xd), np.abs(gd))
+    assert np.all(np.abs(got - want) <= b * h * w * 2.0 ** -24 * size + 2.0 ** -24 * np.abs(want))
