@@ -533,35 +533,28 @@ struct WgradArgs {
   const __nv_bfloat16* grad;  // gradient at the layer output [batch][h][w][cout]
   float* partial;             // per CTA: [3 dy][3 dx][cin][cout]
   int batch, h, w;
-  int rows;    // output rows of a band
+  int rows;    // output rows of a CTA's band
   int tiles;   // bands side by side (128 pixels each)
   int chunks;  // bands over the height
-  int bands;   // of a CTA: 1 or kWgradBands
   int* status;
 };
-
-constexpr int kWgradBands = 2;
-constexpr int kWgradSlots = 4;
 
 template <int CIN, int COUT>
 struct WgradSmem {
   static constexpr uint32_t ROW = 4 * kRowLbo;  // input row: room for 32 channels
   static constexpr uint32_t G_ROW = (COUT / 8) * kRowLbo;
-  static constexpr uint32_t BAND = kWgradSlots * ROW + 2 * G_ROW;
-  static constexpr uint32_t FOLD = 9 * CIN * (COUT + 1) * 4;  // in the place of the bands
-  static constexpr uint32_t USED = kWgradBands * BAND > FOLD ? kWgradBands * BAND : FOLD;
-  // above half an SM's shared memory where a CTA takes all TMEM columns
-  static constexpr uint32_t BYTES = (COUT == 32 && USED < 118 * 1024 ? 118 * 1024 : USED) + 64;
-  static constexpr uint32_t TMEM_COLS = COUT == 32 ? 512 : 256;  // 4 phases x 3 dx x COUT
+  static constexpr uint32_t STAGE = 4 * ROW + 2 * G_ROW;
+  static constexpr uint32_t FOLD = 9 * CIN * (COUT + 1) * 4;  // in the place of the stages
+  static constexpr uint32_t BYTES = (2 * STAGE > FOLD ? 2 * STAGE : FOLD) + 64;
+  static constexpr uint32_t TMEM_COLS = COUT == 32 ? 256 : 128;  // 3 dx x 2 rows x COUT
 };
 
 // Starts the copy of pixels [x, x + n) of an image row of C channels into a
 // staged row: 16-byte pieces, neighbouring threads on neighbouring addresses;
-// zeros outside the image.
+// zeros outside the image and where row is false.
 template <int C>
-__device__ __forceinline__ void wgrad_row_async(const __nv_bfloat16* __restrict__ image, int h,
-                                                int w, int r, int x, int n, uint32_t dst) {
-  const bool row = r >= 0 && r < h;
+__device__ __forceinline__ void wgrad_row_async(const __nv_bfloat16* __restrict__ image, int w,
+                                                bool row, int r, int x, int n, uint32_t dst) {
   const __nv_bfloat16* src = image + (size_t)(row ? r : 0) * w * C;
   for (int i = threadIdx.x; i < n * (C / 8); i += kConvThreads) {
     const int p = i / (C / 8), c8 = i % (C / 8);
@@ -577,16 +570,16 @@ __device__ __forceinline__ void wgrad_row_async(const __nv_bfloat16* __restrict_
 // Both operands are contracted over pixels, so both are MN-major in the staged rows
 // as they lie in memory (16 bytes = 8 channels of a pixel; core matrices of 8 pixels,
 // 128 B apart along K; channel groups kRowLbo apart along M and N): nothing is
-// transposed, and a dx is the same rows dx * 16 bytes on.  The four slots of the row
-// ring are M = 4 x 32 channels: at output row y three of them are dy = 0, 1, 2 and the
-// fourth, which takes row y + 2 meanwhile, gives products that are never read.  Which
-// slot is which dy depends on y mod 4, so each of the four phases has its own three
-// (dx) accumulators of COUT columns.  A step of a CTA is one output row of each of its
-// bands; the next rows are in flight during its MMAs.
+// transposed, and a dx is the same rows dx * 16 bytes on.  A step takes two output
+// rows y, y + 1 (N = 2 x COUT) against the four input rows y - 1 .. y + 2 (M = 4 x 32
+// channels): six of the eight row pairs are the dy = 0, 1, 2 of the two rows, the other
+// two are not read.  The next step's rows are in flight during the MMAs.
 //
-// Bound by the rows' way through shared memory (67 MB for 32 images of 128 x 128 x 32,
-// mostly from L2).  Transposing each row with 2-byte stores and waiting for its MMAs
-// took 147 to 186 us there, this takes 57 to 61.
+// An MMA of K = 16 costs about 75 cycles for any N up to 96 here, so two rows per MMA
+// halve the tensor time; the two rows' windows share no buffer, which leaves one set of
+// accumulators (192 columns) and room for two CTAs per SM.  32 images of 128 x 128 x 32
+// (67 MB, 10 us at the copy rate): 31 to 40 us; one row per step and one CTA of two
+// bands per SM 57 to 61 us; rows transposed with 2-byte stores 147 to 186 us.
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_tc_kernel(const WgradArgs a) {
   using S = WgradSmem<CIN, COUT>;
@@ -595,42 +588,25 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_tc_kernel(const Wg
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t base = smem_u32(smem);
-
-  int y0[kWgradBands], y1[kWgradBands], x0[kWgradBands], npx[kWgradBands];
-  const __nv_bfloat16 *in[kWgradBands], *grad[kWgradBands];
-  int steps = 0;
+  const int q = blockIdx.x / a.tiles, img = q / a.chunks;
+  const int x0 = ((int)blockIdx.x - q * a.tiles) * 128;
+  const int y0 = (q - img * a.chunks) * a.rows, y1 = min(y0 + a.rows, a.h);
+  const int npx = (min(a.w - x0, 128) + 15) / 16 * 16;  // K of a step's MMAs
+  const int steps = (y1 - y0 + 1) / 2;
+  const __nv_bfloat16* in = a.in + (size_t)img * a.h * a.w * CIN;
+  const __nv_bfloat16* grad = a.grad + (size_t)img * a.h * a.w * COUT;
+  auto load = [&](int i) {
+    const uint32_t dst = base + (i & 1) * S::STAGE;
+    const int y = y0 + 2 * i;
 #pragma unroll
-  for (int n = 0; n < kWgradBands; ++n) {
-    const int items = a.tiles * a.chunks * a.batch;
-    const int it = blockIdx.x * a.bands + n;
-    const bool has = n < a.bands && it < items;
-    const int q = has ? it / a.tiles : 0, img = q / a.chunks;
-    x0[n] = has ? (it - q * a.tiles) * 128 : 0;
-    y0[n] = has ? (q - img * a.chunks) * a.rows : 0;
-    y1[n] = has ? min(y0[n] + a.rows, a.h) : 0;
-    npx[n] = (min(a.w - x0[n], 128) + 15) / 16 * 16;  // K of its MMAs
-    in[n] = a.in + (size_t)img * a.h * a.w * CIN;
-    grad[n] = a.grad + (size_t)img * a.h * a.w * COUT;
-    steps = max(steps, y1[n] - y0[n]);
-  }
-  auto slot = [&](int n, int r) { return base + n * S::BAND + ((r + 4) & 3) * S::ROW; };
-  auto gslot = [&](int n, int y) {
-    return base + n * S::BAND + kWgradSlots * S::ROW + (y & 1) * S::G_ROW;
-  };
-  auto load_in = [&](int n, int r) {
-    if (y0[n] < y1[n] && r <= y1[n])
-      wgrad_row_async<CIN>(in[n], a.h, a.w, r, x0[n] - 1, npx[n] + 2, slot(n, r));
-  };
-  auto load_grad = [&](int n, int y) {
-    if (y < y1[n]) wgrad_row_async<COUT>(grad[n], a.h, a.w, y, x0[n], npx[n], gslot(n, y));
-  };
+    for (int k = 0; k < 4; ++k)
+      wgrad_row_async<CIN>(in, a.w, y - 1 + k >= 0 && y - 1 + k < a.h, y - 1 + k, x0 - 1, npx + 2,
+                           dst + k * S::ROW);
 #pragma unroll
-  for (int n = 0; n < kWgradBands; ++n) {
-    load_in(n, y0[n] - 1);
-    load_in(n, y0[n]);
-    load_in(n, y0[n] + 1);
-    load_grad(n, y0[n]);
-  }
+    for (int k = 0; k < 2; ++k)
+      wgrad_row_async<COUT>(grad, a.w, y + k < y1, y + k, x0, npx, dst + 4 * S::ROW + k * S::G_ROW);
+  };
+  load(0);
   asm volatile("cp.async.commit_group;" ::: "memory");
   if (tid == 0) {
     mbar_init(bar, 1);
@@ -642,66 +618,52 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_tc_kernel(const Wg
   tc_fence_after();
   const uint32_t tmem = *tslot;
   const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll 1
-  for (int k = 0; k < 12; ++k) tmem_zero<COUT>(lane_addr + (uint32_t)(k * COUT));
-  tc_fence_before();
-  const uint32_t idesc = umma_idesc_bf16(128, COUT, true);
+  const uint32_t idesc = umma_idesc_bf16(128, 2 * COUT, true);
   bool ok = true;
   for (int i = 0; i < steps; ++i) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     fence_async_smem();
-    __syncthreads();  // rows y - 1 .. y + 1 and the gradient row are staged
+    __syncthreads();  // step i's rows are staged
     if (tid == 0) {
       tc_fence_after();
+      const uint32_t src = base + (i & 1) * S::STAGE;
+      const uint64_t adesc = umma_desc(src, 128, kRowLbo);
+      const uint64_t bdesc = umma_desc(src + 4 * S::ROW, 128, kRowLbo);
+      for (int kk = 0; kk < npx / 16; ++kk)
 #pragma unroll
-      for (int n = 0; n < kWgradBands; ++n) {
-        const int y = y0[n] + i;
-        if (y >= y1[n]) continue;
-        const uint64_t adesc = umma_desc(slot(n, 0), 128, kRowLbo);
-        const uint64_t bdesc = umma_desc(gslot(n, y), 128, kRowLbo);
-        const uint32_t d = tmem + (uint32_t)((y & 3) * 3 * COUT);
-        for (int kk = 0; kk < npx[n] / 16; ++kk)
-#pragma unroll
-          for (int dx = 0; dx < 3; ++dx)
-            umma_bf16(d + dx * COUT, adesc + (uint64_t)(kk * 16 + dx),
-                      bdesc + (uint64_t)(kk * 16), idesc, 1);
-      }
+        for (int dx = 0; dx < 3; ++dx)
+          umma_bf16(tmem + dx * 2 * COUT, adesc + (uint64_t)(kk * 16 + dx),
+                    bdesc + (uint64_t)(kk * 16), idesc, i > 0 || kk > 0);
       umma_commit(bar + (i & 1));
     }
-    // the previous step's MMAs have read the slots that the next rows take
+    // step i - 1's MMAs have read the stage that step i + 1 takes
     if (i > 0) ok = mbar_wait(bar + ((i - 1) & 1), ((i - 1) >> 1) & 1) && ok;
-    if (i + 1 < steps) {
-#pragma unroll
-      for (int n = 0; n < kWgradBands; ++n) {
-        load_in(n, y0[n] + i + 2);
-        load_grad(n, y0[n] + i + 1);
-      }
-    }
+    if (i + 1 < steps) load(i + 1);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  if (steps > 0) ok = mbar_wait(bar + ((steps - 1) & 1), ((steps - 1) >> 1) & 1) && ok;
+  ok = mbar_wait(bar + ((steps - 1) & 1), ((steps - 1) >> 1) & 1) && ok;
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   tc_fence_after();
-  __syncthreads();  // every MMA has completed: the rows' place takes the sums
-  // warp = slot, lane = ci.  Slot s holds dy at phase p = s + 1 - dy (mod 4).  The
-  // warps take the taps in turn, four groups of them in four rounds, so each tap's
-  // four shares are added in a fixed order.
+  __syncthreads();  // every MMA has completed: the stages' place takes the sums
+  // warp = input row of the window, lane = ci.  Row s and output row j (0, 1) of the
+  // step are dy = s - j: first the shares of j = 0, then those of j = 1 on top.
   float* fold = reinterpret_cast<float*>(smem);
 #pragma unroll 1
-  for (int round = 0; round < 4; ++round) {
+  for (int j = 0; j < 2; ++j) {
+    const int dy = warp - j;
+    if (dy >= 0 && dy < 3) {
 #pragma unroll 1
-    for (int tap = (warp + round) & 3; tap < 9; tap += 4) {
-      const int dy = tap / 3, dx = tap - dy * 3;
-      float v[COUT];
-      const uint32_t col = (uint32_t)((((warp + 5 - dy) & 3) * 3 + dx) * COUT);
-      if constexpr (COUT == 32)
-        tmem_ld32(lane_addr + col, v);
-      else
-        tmem_ld16(lane_addr + col, v);
-      if (lane < CIN) {
-        float* f = fold + (tap * CIN + lane) * (COUT + 1);
+      for (int dx = 0; dx < 3; ++dx) {
+        float v[COUT];
+        if constexpr (COUT == 32)
+          tmem_ld32(lane_addr + (uint32_t)((dx * 2 + j) * COUT), v);
+        else
+          tmem_ld16(lane_addr + (uint32_t)((dx * 2 + j) * COUT), v);
+        if (lane < CIN) {
+          float* f = fold + ((dy * 3 + dx) * CIN + lane) * (COUT + 1);
 #pragma unroll
-        for (int co = 0; co < COUT; ++co) f[co] = round == 0 ? v[co] : f[co] + v[co];
+          for (int co = 0; co < COUT; ++co) f[co] = j == 0 ? v[co] : f[co] + v[co];
+        }
       }
     }
     __syncthreads();

@@ -50,9 +50,8 @@ cudaError_t launch_wgrad(const WgradArgs& a, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  const int items = a.tiles * a.chunks * a.batch;
   conv3x3_wgrad_tc_kernel<CIN, COUT>
-      <<<(items + a.bands - 1) / a.bands, kConvThreads, S::BYTES, st>>>(a);
+      <<<a.tiles * a.chunks * a.batch, kConvThreads, S::BYTES, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -185,7 +184,7 @@ int sb_learned_wgrad(const void* in, const void* grad, float* partial, size_t pa
     return lcuda(cudaErrorInvalidConfiguration);
   WgradArgs a{(const __nv_bfloat16*)in, (const __nv_bfloat16*)grad, partial, batch, h, w,
               rows_per_cta, (w + 127) / 128, (h + rows_per_cta - 1) / rows_per_cta,
-              nctas > 148 ? kWgradBands : 1, d_status};
+              d_status};
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e;
   if (cin == 16 && cout == 32) e = launch_wgrad<16, 32>(a, st);
@@ -193,8 +192,8 @@ int sb_learned_wgrad(const void* in, const void* grad, float* partial, size_t pa
   else if (cin == 32 && cout == 16) e = launch_wgrad<32, 16>(a, st);
   else e = launch_wgrad<16, 16>(a, st);
   if (e != cudaSuccess) return lcuda(e);
-  const int n = 9 * cin * cout, ctas = ((int)nctas + a.bands - 1) / a.bands;
-  wgrad_reduce_kernel<<<(n + 31) / 32, 256, 0, st>>>(partial, ctas, n, dw);
+  const int n = 9 * cin * cout;
+  wgrad_reduce_kernel<<<(n + 31) / 32, 256, 0, st>>>(partial, (int)nctas, n, dw);
   return lcuda(cudaGetLastError());
 }
 
