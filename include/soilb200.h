@@ -519,6 +519,11 @@ const char* sb_learned_last_error(void);
 int sb_learned_conv(const void* in, void* out, const void* wpk, const void* mask, int batch, int h,
                     int w, int cin, int cout, int relu, int out_f32, int rows_per_cta,
                     int* d_status, void* stream);
+/* The four layers' f32 weights [3][3][cin][cout] as packed bf16 operands, one
+ * after another (9*cin*cout each), of the convolution or (backward != 0) of its
+ * data gradient. */
+int sb_learned_pack(const float* w0, const float* w1, const float* w2, const float* w3,
+                    int backward, void* out, void* stream);
 /* dW[3][3][cin][cout] (f32) of a layer from its input and output gradient;
  * partial: ceil(w/128)*ceil(h/rows)*batch*3*128*cout floats of scratch. */
 int sb_learned_wgrad(const void* in, const void* grad, float* partial, size_t partial_floats,

@@ -527,6 +527,40 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_rot_kernel(const ConvArg
   if (warp == 0) tmem_free(tmem, S::TMEM_COLS);
 }
 
+// ------------------------------------------------------- packed weights
+// The network's four layers (channels 16-32-32-32-16), one after another.
+constexpr int kNetLayers = 4;
+struct PackArgs {
+  const float* w[kNetLayers];  // [3][3][ci][co]
+  __nv_bfloat16* out;
+};
+
+// W[3][3][ci][co] -> the canonical K-major operand of each tap (rows n = output
+// channel, k = input channel; 8 x 8 core matrices, (n / 8, k / 8) blocks).
+// backward: of the data gradient's weights W'[dy][dx][co][ci] = W[2-dy][2-dx][ci][co].
+// All layers in one launch: bound by launches, not by its 166 KB (as a gather, a cast
+// and two flips per layer: 28 launches, 81 us of kernels in a training step).
+__global__ void __launch_bounds__(256) learned_pack_kernel(const PackArgs a, int backward) {
+  constexpr int kCh[kNetLayers + 1] = {16, 32, 32, 32, 16};
+  int i = blockIdx.x * 256 + threadIdx.x;
+  __nv_bfloat16* out = a.out + i;
+#pragma unroll
+  for (int l = 0; l < kNetLayers; ++l) {
+    const int ci = kCh[l], co = kCh[l + 1], block = ci * co;
+    if (i < 0 || i >= 9 * block) {
+      i -= 9 * block;  // of a later layer, or (negative) already done
+      continue;
+    }
+    const int kdim = backward ? co : ci;
+    const int tap = i / block, off = i - tap * block, core = off >> 6;
+    const int n = core / (kdim >> 3) * 8 + ((off >> 3) & 7);
+    const int k = core % (kdim >> 3) * 8 + (off & 7);
+    const int src = backward ? ((8 - tap) * ci + n) * co + k : (tap * ci + k) * co + n;
+    *out = __float2bfloat16_rn(a.w[l][src]);
+    return;
+  }
+}
+
 // ----------------------------------------------------------- weight grad
 struct WgradArgs {
   const __nv_bfloat16* in;    // layer input [batch][h][w][cin]

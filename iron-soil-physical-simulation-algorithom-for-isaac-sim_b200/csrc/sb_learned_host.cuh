@@ -170,6 +170,16 @@ int sb_learned_conv(const void* in, void* out, const void* wpk, const void* mask
   return lcuda(e);
 }
 
+int sb_learned_pack(const float* w0, const float* w1, const float* w2, const float* w3,
+                    int backward, void* out, void* stream) {
+  if (!w0 || !w1 || !w2 || !w3 || !out)
+    return lfail(SB_ERR_BAD_ARG, "[soilb200] pack: bad arguments");
+  const int n = 9 * (16 * 32 + 32 * 32 + 32 * 32 + 32 * 16);
+  learned_pack_kernel<<<n / 256, 256, 0, (cudaStream_t)stream>>>(
+      PackArgs{{w0, w1, w2, w3}, (__nv_bfloat16*)out}, backward);
+  return lcuda(cudaGetLastError());
+}
+
 // partial must hold ceil(w/128) * ceil(h/rows) * batch * 3 * 128 * cout floats.
 int sb_learned_wgrad(const void* in, const void* grad, float* partial, size_t partial_floats,
                      float* dw, int batch, int h, int w, int cin, int cout, int rows_per_cta,

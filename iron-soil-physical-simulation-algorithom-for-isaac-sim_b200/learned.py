@@ -84,14 +84,32 @@ class ReposeNet:
                          for ci, co in LAYERS]
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
 
+    def _pack(self, backward: bool):
+        """Both directions' packed BF16 operands in one kernel; None where the
+        weights are not the network's own float32 device tensors."""
+        torch = _torch()
+        if len(self.weights) != len(LAYERS) or any(
+                w.dtype != torch.float32 or w.device != self.device or w.requires_grad
+                or tuple(w.shape) != (3, 3, *c) for w, c in zip(self.weights, LAYERS)):
+            return None
+        src = [w.contiguous() for w in self.weights]
+        sizes = [9 * ci * co for ci, co in LAYERS]
+        out = torch.empty(sum(sizes), dtype=torch.bfloat16, device=self.device)
+        with torch.cuda.device(self.device):
+            _ok(_lib.load().sb_learned_pack(
+                *(w.data_ptr() for w in src), int(backward), out.data_ptr(),
+                torch.cuda.current_stream(self.device).cuda_stream), "pack")
+        return list(out.split(sizes))
+
     def packed(self):
         torch = _torch()
-        return [w.reshape(-1)[i].to(torch.bfloat16) for w, i in zip(self.weights, self._fwd_idx)]
+        return self._pack(False) or [w.reshape(-1)[i].to(torch.bfloat16)
+                                     for w, i in zip(self.weights, self._fwd_idx)]
 
     def packed_backward(self):
         torch = _torch()
-        return [flip_transpose(w).reshape(-1)[i].to(torch.bfloat16)
-                for w, i in zip(self.weights, self._bwd_idx)]
+        return self._pack(True) or [flip_transpose(w).reshape(-1)[i].to(torch.bfloat16)
+                                    for w, i in zip(self.weights, self._bwd_idx)]
 
     def numpy_weights(self):
         return [w.detach().cpu().numpy().astype(np.float64) for w in self.weights]

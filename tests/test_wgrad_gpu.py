@@ -31,3 +31,19 @@ def test_wgrad_band_edges(b, h, w, rows, cin, cout):
     want = L.conv3x3_wgrad(xd, gd)
     size = L.conv3x3_wgrad(np.abs(xd), np.abs(gd))
     assert np.all(np.abs(got - want) <= b * h * w * 2.0 ** -24 * size + 2.0 ** -24 * np.abs(want))
+
+
+def test_packed_weights_are_the_gathered_ones():
+    net = ln.ReposeNet(seed=4)
+    for w in net.weights:  # padded channels too, and values that round
+        w.copy_(torch.randn(w.shape, generator=torch.Generator().manual_seed(w.numel())))
+    for li, (ci, co) in enumerate(ln.LAYERS):
+        w = net.weights[li].cpu()
+        fwd = w.reshape(-1)[torch.as_tensor(ln.pack_index(ci, co))].to(torch.bfloat16)
+        bwd = ln.flip_transpose(w).reshape(-1)[torch.as_tensor(ln.pack_index(co, ci))]
+        assert torch.equal(net.packed()[li].cpu(), fwd)
+        assert torch.equal(net.packed_backward()[li].cpu(), bwd.to(torch.bfloat16))
+    # weights of another form take the gather
+    want = net.packed()
+    net.weights = [w.double() for w in net.weights]
+    assert all(torch.equal(g, w) for g, w in zip(net.packed(), want))
