@@ -125,9 +125,12 @@ class ReposeNet:
 
 
 def conv_rows(b: int, h: int, w: int) -> int:
-    """Rows per CTA: about one wave of 4 resident CTAs on each of 148 SMs."""
-    tiles = (w + 127) // 128
-    return int(min(32, max(4, -(-b * h * tiles // (148 * 4)))))
+    """Rows per CTA: the fewest (4 to 32) that make one wave of 3 CTAs on each
+    of 148 SMs.  32 -> 32 channels, 32 x 128 x 128 and 701 x 701: 26 us with 10
+    rows (416 and 426 CTAs), 28 with 8 (4 per SM), 32 with 7 (608 CTAs, a last
+    wave of 16), 30 with 13."""
+    bands = max(1, 148 * 3 // (b * ((w + 127) // 128)))
+    return int(min(32, max(4, -(-h // bands))))
 
 
 def conv(x, wpk, cin: int, cout: int, *, relu: bool, out_f32: bool | int = False, mask=None,

@@ -47,3 +47,23 @@ def test_packed_weights_are_the_gathered_ones():
     want = net.packed()
     net.weights = [w.double() for w in net.weights]
     assert all(torch.equal(g, w) for g, w in zip(net.packed(), want))
+
+
+@pytest.mark.parametrize("rot", ["0", "1"])
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (32, 16), (16, 32), (32, 32)])
+@pytest.mark.parametrize("w", [1, 3, 4, 127, 130])
+def test_bf16_rows_are_the_rounded_f32_rows(monkeypatch, w, cin, cout, masked, rot):
+    """The exchanged 16-byte pieces of a BF16 row against the FP32 output, which
+    each thread writes for its own pixel: the same values, rounded."""
+    monkeypatch.setenv("SOILB200_CONV_ROT", rot)
+    rng = np.random.default_rng(w + cin + 2 * cout)
+    x, m = _bf16(rng, 2, 5, w, cin).cuda(), _bf16(rng, 2, 5, w, cout).cuda()
+    wpk = _bf16(rng, 9 * cin * cout).cuda()
+    mask = m if masked else None
+    for relu in (False, True):
+        f32 = ln.conv(x, wpk, cin, cout, relu=relu, out_f32=True, mask=mask)
+        out = ln.conv(x, wpk, cin, cout, relu=relu, mask=mask)
+        assert torch.equal(out, f32.to(torch.bfloat16))
+        if masked:
+            assert not torch.any(out[~(m > 0)])
