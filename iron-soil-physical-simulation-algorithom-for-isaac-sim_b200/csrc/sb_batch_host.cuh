@@ -651,10 +651,11 @@ int sb_batch_label(sb_batch* bt, const sb_label_params* p, sb_label_stats* out) 
     c.Q = std::ldexp(1.0, -d.height_exponent);
     c.datum = d.datum_m;
     c.release_latches = 0;  // no latches in a batch
+    c.yield = yield_constants(c);
     const long long base = bt->base[i];
     const int tiles = c.tiles_x * ((d.ny + kLabelTile - 1) / kLabelTile);
     LabelOut* lo = bt->lab_out + i;
-    label_init_local_kernel<true><<<tiles, kLabelInitThreads, 0, bt->stream>>>(
+    label_init_local_kernel<true><<<tiles, kLabelInitThreads<true>, 0, bt->stream>>>(
         c, bt->b + base, bt->z + base, bt->h[0] + base, bt->h[1] + base, bt->qx[0] + base,
         bt->qx[1] + base, bt->qy[0] + base, bt->qy[1] + base, &bt->d_ctl[i].k, bt->lab_parent,
         bt->lab_slope, bt->lab_severity, bt->lab_zero_i, bt->lab_zero_d, bt->lab_zero_d,

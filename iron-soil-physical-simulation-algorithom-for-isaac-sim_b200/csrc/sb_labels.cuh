@@ -29,21 +29,36 @@
 
 #include "sb_common.cuh"
 #include "sb_fv.cuh"
+#include "sb_ledger.cuh"
 
 namespace sb {
 
 constexpr int kLabelTile = 32;
-// Threads of the yield/labelling tile kernel: 16 warps per 32x32 tile (two
-// cells per thread) and 3 tiles per SM; measured with the FP64 yield (now the
-// parity path only; the fixed-point path's yield is float32), 12 warps per
-// tile (4 tiles per SM) were 1.3 % slower on the whole 701^2 step, 8 warps
-// 0.1 % slower still.
-constexpr int kLabelInitThreads = 512;
+// Threads of the yield/labelling tile kernel.  FP64: 16 warps per 32x32 tile (two
+// cells per thread) and 3 tiles per SM; 12 warps per tile (4 tiles per SM) were
+// 1.3 % slower on the whole 701^2 step, 8 warps 0.1 % slower still.  Fixed point: a
+// thread owns four neighbours of a row.
+template <bool FX>
+constexpr int kLabelInitThreads = FX ? kLabelTile * kLabelTile / 4 : 512;
 // Fixed-point units of the per-root sums.  2^32 keeps the int64 sums free of
 // overflow up to 2^24 cells with slopes < pi/2 rad and failure depths < 8 m
 // (1.7e7 * 8 * 6 * 2^32 < 2^63), at a resolution of 2.3e-10.
 constexpr double kExcessScale = 4294967296.0;     // 2^32 per radian
 constexpr double kVolumeScaleFp64 = 4294967296.0;  // 2^32 per (m * w6)
+
+// Fixed-point yield constants in float32, each one rounding of its double
+// expression: gradient scales {Q / (2 dx), Q / dx} and {Q / (2 dy), Q / dy},
+// the quantum, the mobilization depth, density * gravity, cohesion, the start
+// and stop tangents, their difference and the dry tolerance.
+struct YieldF {
+  float sx0, sx1, sy0, sy1;
+  float Q, depth, rg, coh, ts, tp, dts, dry;
+  // A gradient below this is stable against both angles whatever the layer:
+  // 1e-5 under the smaller tangent, where the margins' float32 rounding stays
+  // below 1e-6 of the friction term; negative (never) for parameters of other
+  // signs.
+  float calm;
+};
 
 struct LabelConst {
   int ny, nx, pitch, tiles_x, connectivity;
@@ -52,6 +67,7 @@ struct LabelConst {
   double Q, datum;
   int release_latches;
   int tile_size, frontier_tiles_x;  // frontier tile geometry for seeding
+  YieldF yield;
 };
 
 // Per-root accumulators (flat index = root).
@@ -92,26 +108,13 @@ __device__ __forceinline__ double free_surface_diff(const typename FvTypes<FX>::
   }
 }
 
-// Fixed-point yield constants in float32, each one rounding of its double
-// expression: gradient scales {Q / (2 dx), Q / dx} and {Q / (2 dy), Q / dy},
-// the quantum, the mobilization depth, density * gravity, cohesion, the start
-// and stop tangents, their difference and the dry tolerance.
-struct YieldF {
-  float sx[2], sy[2];
-  float Q, depth, rg, coh, ts, tp, dts, dry;
-  // A gradient below this is stable against both angles whatever the layer:
-  // 1e-5 under the smaller tangent, where the margins' float32 rounding stays
-  // below 1e-6 of the friction term; negative (never) for parameters of other
-  // signs.
-  float calm;
-};
-
-__device__ __forceinline__ YieldF yield_constants(const LabelConst& c) {
+// On the host: in the kernel, its four divisions a thread cost as much as the cells.
+inline YieldF yield_constants(const LabelConst& c) {
   YieldF y;
-  y.sx[0] = (float)(c.Q / (2.0 * c.dx));
-  y.sx[1] = (float)(c.Q / c.dx);
-  y.sy[0] = (float)(c.Q / (2.0 * c.dy));
-  y.sy[1] = (float)(c.Q / c.dy);
+  y.sx0 = (float)(c.Q / (2.0 * c.dx));
+  y.sx1 = (float)(c.Q / c.dx);
+  y.sy0 = (float)(c.Q / (2.0 * c.dy));
+  y.sy1 = (float)(c.Q / c.dy);
   y.Q = (float)c.Q;
   y.depth = (float)c.mob_depth;
   y.rg = (float)(c.density * c.gravity);
@@ -121,7 +124,7 @@ __device__ __forceinline__ YieldF yield_constants(const LabelConst& c) {
   y.dts = (float)(c.tan_start - c.tan_stop);
   y.dry = (float)c.dry;
   y.calm = y.coh >= 0.f && y.rg > 0.f && y.ts > 0.f && y.tp > 0.f && y.depth > 0.f
-               ? fminf(y.ts, y.tp) * (1.f - 1.0e-5f)
+               ? std::fmin(y.ts, y.tp) * (1.f - 1.0e-5f)
                : -1.f;
   return y;
 }
@@ -202,8 +205,163 @@ __device__ __forceinline__ void local_ccl(int* lab, int connectivity, int gy0, i
 }
 
 
+__device__ __forceinline__ void label_clear_root(const LabelRoots& roots, long long flat) {
+  roots.count[flat] = 0;
+  roots.area6[flat] = 0;
+  roots.volume[flat] = 0;
+  roots.exc_start[flat] = 0;
+  roots.exc_stop[flat] = 0;
+  roots.max_exc_start[flat] = 0;
+  roots.max_exc_stop[flat] = 0;
+  roots.prev_overlap[flat] = 0;
+}
+
+// Whether the set latch of cell (r, col) is released (mob: its mobile depth).
+__device__ __forceinline__ bool latch_settles(const LabelConst& c, double mob, double qx, double qy,
+                                              int r, int col, long long flat, bool settled,
+                                              const double* __restrict__ export_cum,
+                                              const double* __restrict__ export_base) {
+  double speed = 0.0;
+  if (mob > c.dry) {
+    const double vx = qx / mob, vy = qy / mob;
+    speed = sqrt(vx * vx + vy * vy);
+  }
+  const double w = (double)vertex_weight6(r, col, c.ny, c.nx) * (c.dx * c.dy / 6.0);
+  const bool resolved = (export_cum[flat] - export_base[flat]) > c.dry * w;
+  return speed <= c.activity_speed && (resolved || settled);
+}
+
+// Fixed-point yield of this thread's four neighbours of a row of the tile, in float32
+// throughout (the ledger and the exchange sums are the only FP64 work of the
+// fixed-point path).  Writes slope, severity, parent and lab; returns whether a cell
+// is unstable.
+//
+// 24 B per cell (61 us at 4096^2 and the measured copy rate).  One cell per thread and
+// turn, 64-bit differences and the constants' divisions in every thread took 207 us
+// there; 16-byte words, 32-bit differences (64-bit ones where they wrap) and host
+// constants 124 us (6 CTAs per SM at 40 registers: 163).
+__device__ __forceinline__ int yield_quad_fx(
+    const LabelConst& c, const int32_t* __restrict__ b, const int32_t* __restrict__ z,
+    const int32_t* __restrict__ h, const float* __restrict__ qx, const float* __restrict__ qy,
+    int gy0, int gx0, int* lab, int* __restrict__ parent, float* __restrict__ slope_out,
+    float* __restrict__ severity_out, int* __restrict__ latch,
+    const double* __restrict__ export_cum, const double* __restrict__ export_base,
+    const LabelRoots& roots) {
+  const int li = threadIdx.x * 4;
+  const int r = gy0 + li / kLabelTile, col = gx0 + li % kLabelTile;
+  const int n = r < c.ny ? min(c.nx - col, 4) : 0;
+  if (n <= 0) {
+    *reinterpret_cast<int4*>(lab + li) = make_int4(-1, -1, -1, -1);
+    return 0;
+  }
+  const YieldF& yf = c.yield;
+  const unsigned gi = (unsigned)r * (unsigned)c.pitch + (unsigned)col;
+  const unsigned dn = r > 0 ? gi - (unsigned)c.pitch : gi;
+  const unsigned up = r + 1 < c.ny ? gi + (unsigned)c.pitch : gi;
+  // the words past nx are the row's padding
+  const int4 b4 = *reinterpret_cast<const int4*>(b + gi), h4 = *reinterpret_cast<const int4*>(h + gi);
+  const int4 bd = *reinterpret_cast<const int4*>(b + dn), hd = *reinterpret_cast<const int4*>(h + dn);
+  const int4 bu = *reinterpret_cast<const int4*>(b + up), hu = *reinterpret_cast<const int4*>(h + up);
+  const int4 z4 = *reinterpret_cast<const int4*>(z + gi);
+  const unsigned gl = col > 0 ? gi - 1 : gi, gr = col + n < c.nx ? gi + n : gi + n - 1;
+  const int bl = b[gl], hl = h[gl], br = b[gr], hr = h[gr];
+  const int bq[4] = {b4.x, b4.y, b4.z, b4.w}, hq[4] = {h4.x, h4.y, h4.z, h4.w};
+  const int zq[4] = {z4.x, z4.y, z4.z, z4.w};
+  const int bdn[4] = {bd.x, bd.y, bd.z, bd.w}, hdn[4] = {hd.x, hd.y, hd.z, hd.w};
+  const int bup[4] = {bu.x, bu.y, bu.z, bu.w}, hup[4] = {hu.x, hu.y, hu.z, hu.w};
+  int over = 0;  // sign bit: a 32-bit sum or difference wrapped
+  int s[6];      // b + h of the cells and of their neighbours left and right
+  s[0] = wrap_add(bl, hl, over);
+  const int beyond = wrap_add(br, hr, over);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) s[k + 1] = k < n ? wrap_add(bq[k], hq[k], over) : beyond;
+  s[5] = beyond;
+  float fdx[4], fdy[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    fdx[k] = fdy[k] = 0.f;
+    if (k >= n) continue;
+    fdx[k] = (float)wrap_sub(s[k + 2], s[k], over);
+    fdy[k] = (float)wrap_sub(wrap_add(bup[k], hup[k], over), wrap_add(bdn[k], hdn[k], over), over);
+  }
+  if (over < 0) {
+    long long w[6];
+    w[0] = (long long)bl + hl;
+    w[5] = (long long)br + hr;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k + 1] = k < n ? (long long)bq[k] + hq[k] : w[5];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      fdx[k] = (float)(w[k + 2] - w[k]);
+      fdy[k] = (float)(((long long)bup[k] + hup[k]) - ((long long)bdn[k] + hdn[k]));
+    }
+  }
+  const bool iny = r > 0 && r + 1 < c.ny;
+  float slope[4], sev[4];
+  unsigned um = 0, settled = 0xfu;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const bool inx = col + k > 0 && col + k + 1 < c.nx;
+    const float gx = fdx[k] * (inx ? yf.sx0 : yf.sx1);
+    const float gy = fdy[k] * (iny ? yf.sy0 : yf.sy1);
+    const float mag = sqrtf(gx * gx + gy * gy);
+    slope[k] = atan_as4449(mag);
+    sev[k] = 0.f;
+    if (!(mag < yf.calm) && k < n) {  // nearly all cells are calm: no roots, no divisions
+      const long long dq = (long long)bq[k] - (long long)zq[k];
+      const float layer = fminf((float)(dq > 0 ? dq : 0) * yf.Q, yf.depth);
+      const float norm = sqrtf(1.0f + mag * mag);
+      const float drive = yf.rg * layer * mag / norm;
+      const float normal = yf.rg * layer / norm;
+      const float start_margin = drive - (yf.coh + normal * yf.ts);
+      const float stop_margin = drive - (yf.coh + normal * yf.tp);
+      sev[k] = fminf(fmaxf(stop_margin / fmaxf(normal * yf.dts, 1.0e-12f), 0.f), 1.f);
+      if (layer > yf.dry && start_margin > 0.f) um |= 1u << k;
+      if (!(stop_margin <= 0.f)) settled &= ~(1u << k);
+    }
+  }
+  const long long flat = (long long)r * c.nx + col;
+  int par[4], lb[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    par[k] = (um >> k) & 1u ? (int)flat + k : -1;
+    lb[k] = (um >> k) & 1u ? li + k : -1;
+  }
+  *reinterpret_cast<int4*>(lab + li) = make_int4(lb[0], lb[1], lb[2], lb[3]);
+  int lt[4] = {0, 0, 0, 0};
+  if ((c.nx & 3) == 0) {  // rows of the outputs start on 16 bytes
+    *reinterpret_cast<float4*>(slope_out + flat) = make_float4(slope[0], slope[1], slope[2], slope[3]);
+    *reinterpret_cast<float4*>(severity_out + flat) = make_float4(sev[0], sev[1], sev[2], sev[3]);
+    *reinterpret_cast<int4*>(parent + flat) = make_int4(par[0], par[1], par[2], par[3]);
+    if (c.release_latches) {
+      const int4 l4 = *reinterpret_cast<const int4*>(latch + flat);
+      lt[0] = l4.x, lt[1] = l4.y, lt[2] = l4.z, lt[3] = l4.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k >= n) continue;
+      slope_out[flat + k] = slope[k];
+      severity_out[flat + k] = sev[k];
+      parent[flat + k] = par[k];
+      if (c.release_latches) lt[k] = latch[flat + k];
+    }
+  }
+  for (unsigned m = um; m; m &= m - 1) label_clear_root(roots, flat + __ffs(m) - 1);
+  // a latch that is already released stays released: only set latches need the
+  // speed and export test
+  if (lt[0] | lt[1] | lt[2] | lt[3])
+#pragma unroll 1
+    for (int k = 0; k < n; ++k)
+      if (latch[flat + k] != 0 &&
+          latch_settles(c, (double)h[gi + k] * c.Q, (double)qx[gi + k], (double)qy[gi + k], r,
+                        col + k, flat + k, (settled >> k) & 1u, export_cum, export_base))
+        latch[flat + k] = 0;
+  return um != 0;
+}
+
 template <bool FX>
-__global__ void __launch_bounds__(kLabelInitThreads, 3)
+__global__ void __launch_bounds__(kLabelInitThreads<FX>, FX ? 4 : 3)
     label_init_local_kernel(const LabelConst c, const typename FvTypes<FX>::B* __restrict__ b,
                             const typename FvTypes<FX>::B* __restrict__ z,
                             const typename FvTypes<FX>::H* __restrict__ h0,
@@ -216,58 +374,28 @@ __global__ void __launch_bounds__(kLabelInitThreads, 3)
                             typename FvTypes<FX>::R* __restrict__ severity_out,
                             int* __restrict__ latch, const double* __restrict__ export_cum,
                             const double* __restrict__ export_base, LabelRoots roots) {
-  __shared__ int lab[kLabelTile * kLabelTile];
+  __shared__ __align__(16) int lab[kLabelTile * kLabelTile];
   const int tx = blockIdx.x % c.tiles_x, ty = blockIdx.x / c.tiles_x;
   const int gx0 = tx * kLabelTile, gy0 = ty * kLabelTile;
   const int P = ctl->parity;  // buffer holding the current mobile state
   const typename FvTypes<FX>::H* h = P ? h1 : h0;
   const typename FvTypes<FX>::R* qx = P ? qx1 : qx0;
   const typename FvTypes<FX>::R* qy = P ? qy1 : qy0;
-  const YieldF yf = yield_constants(c);
   int any = 0;
-  for (int li = threadIdx.x; li < kLabelTile * kLabelTile; li += kLabelInitThreads) {
-    const int ly = li / kLabelTile, lx = li % kLabelTile;
-    const int r = gy0 + ly, col = gx0 + lx;
-    int u = 0;
-    if (r < c.ny && col < c.nx) {
-      const size_t gi = (size_t)r * c.pitch + col;
-      const long long flat = (long long)r * c.nx + col;
-      const int cl = col > 0 ? col - 1 : col, cr = col + 1 < c.nx ? col + 1 : col;
-      const int rd = r > 0 ? r - 1 : r, ru = r + 1 < c.ny ? r + 1 : r;
-      const bool inx = col > 0 && col + 1 < c.nx, iny = r > 0 && r + 1 < c.ny;
-      double mob;
-      bool settled;  // stop margin <= 0
-      if constexpr (FX) {
-        // float32 throughout (the ledger and the exchange sums are the only
-        // FP64 work of the fixed-point path)
-        const long long dxq = ((long long)b[(size_t)r * c.pitch + cr] + h[(size_t)r * c.pitch + cr]) -
-                              ((long long)b[(size_t)r * c.pitch + cl] + h[(size_t)r * c.pitch + cl]);
-        const long long dyq = ((long long)b[(size_t)ru * c.pitch + col] + h[(size_t)ru * c.pitch + col]) -
-                              ((long long)b[(size_t)rd * c.pitch + col] + h[(size_t)rd * c.pitch + col]);
-        // (the 32-bit conversion rounds alike and is four times as fast)
-        const float gx = ((int)dxq == dxq ? (float)(int)dxq : (float)dxq) *
-                         (inx ? yf.sx[0] : yf.sx[1]);
-        const float gy = ((int)dyq == dyq ? (float)(int)dyq : (float)dyq) *
-                         (iny ? yf.sy[0] : yf.sy[1]);
-        const float mag = sqrtf(gx * gx + gy * gy);
-        const long long dq = (long long)b[gi] - (long long)z[gi];
-        mob = (double)h[gi] * c.Q;
-        slope_out[flat] = atan_as4449(mag);
-        float sev = 0.f;
-        settled = true;
-        if (!(mag < yf.calm)) {  // nearly all cells are calm: no roots, no divisions
-          const float layer = fminf((float)(dq > 0 ? dq : 0) * yf.Q, yf.depth);
-          const float norm = sqrtf(1.0f + mag * mag);
-          const float drive = yf.rg * layer * mag / norm;
-          const float normal = yf.rg * layer / norm;
-          const float start_margin = drive - (yf.coh + normal * yf.ts);
-          const float stop_margin = drive - (yf.coh + normal * yf.tp);
-          sev = fminf(fmaxf(stop_margin / fmaxf(normal * yf.dts, 1.0e-12f), 0.f), 1.f);
-          u = (layer > yf.dry && start_margin > 0.f) ? 1 : 0;
-          settled = stop_margin <= 0.f;
-        }
-        severity_out[flat] = sev;
-      } else {
+  if constexpr (FX) {
+    any = yield_quad_fx(c, b, z, h, qx, qy, gy0, gx0, lab, parent, slope_out, severity_out, latch,
+                        export_cum, export_base, roots);
+  } else {
+    for (int li = threadIdx.x; li < kLabelTile * kLabelTile; li += kLabelInitThreads<FX>) {
+      const int ly = li / kLabelTile, lx = li % kLabelTile;
+      const int r = gy0 + ly, col = gx0 + lx;
+      int u = 0;
+      if (r < c.ny && col < c.nx) {
+        const size_t gi = (size_t)r * c.pitch + col;
+        const long long flat = (long long)r * c.nx + col;
+        const int cl = col > 0 ? col - 1 : col, cr = col + 1 < c.nx ? col + 1 : col;
+        const int rd = r > 0 ? r - 1 : r, ru = r + 1 < c.ny ? r + 1 : r;
+        const bool inx = col > 0 && col + 1 < c.nx, iny = r > 0 && r + 1 < c.ny;
         const double denx = inx ? 2.0 * c.dx : c.dx;
         const double deny = iny ? 2.0 * c.dy : c.dy;
         const double gx = free_surface_diff<FX>(b, h, (size_t)r * c.pitch + cr,
@@ -276,7 +404,7 @@ __global__ void __launch_bounds__(kLabelInitThreads, 3)
                                                 (size_t)rd * c.pitch + col, c.Q) / deny;
         const double mag = sqrt(gx * gx + gy * gy);
         const double layer = fmin(fmax(b[gi] - z[gi], 0.0), c.mob_depth);
-        mob = h[gi];
+        const double mob = h[gi];
         const double norm = sqrt(1.0 + mag * mag);
         const double drive = c.density * c.gravity * layer * mag / norm;
         const double normal = c.density * c.gravity * layer / norm;
@@ -286,34 +414,19 @@ __global__ void __launch_bounds__(kLabelInitThreads, 3)
         slope_out[flat] = atan(mag);
         severity_out[flat] = sev;
         u = (layer > c.dry && start_margin > 0.0) ? 1 : 0;
-        settled = stop_margin <= 0.0;
+        const bool settled = stop_margin <= 0.0;
+        parent[flat] = u ? (int)flat : -1;
+        if (u) label_clear_root(roots, flat);
+        // a latch that is already released stays released: only set latches
+        // need the speed and export test
+        if (c.release_latches && latch[flat] != 0 &&
+            latch_settles(c, mob, (double)qx[gi], (double)qy[gi], r, col, flat, settled, export_cum,
+                          export_base))
+          latch[flat] = 0;
       }
-      parent[flat] = u ? (int)flat : -1;
-      if (u) {
-        roots.count[flat] = 0;
-        roots.area6[flat] = 0;
-        roots.volume[flat] = 0;
-        roots.exc_start[flat] = 0;
-        roots.exc_stop[flat] = 0;
-        roots.max_exc_start[flat] = 0;
-        roots.max_exc_stop[flat] = 0;
-        roots.prev_overlap[flat] = 0;
-      }
-      // a latch that is already released stays released: only set latches
-      // need the speed and export test
-      if (c.release_latches && latch[flat] != 0) {
-        double speed = 0.0;
-        if (mob > c.dry) {
-          const double vx = (double)qx[gi] / mob, vy = (double)qy[gi] / mob;
-          speed = sqrt(vx * vx + vy * vy);
-        }
-        const double w = (double)vertex_weight6(r, col, c.ny, c.nx) * (c.dx * c.dy / 6.0);
-        const bool resolved = (export_cum[flat] - export_base[flat]) > c.dry * w;
-        if (speed <= c.activity_speed && (resolved || settled)) latch[flat] = 0;
-      }
+      lab[li] = u ? li : -1;
+      any |= u;
     }
-    lab[li] = u ? li : -1;
-    any |= u;
   }
   if (!__syncthreads_or(any)) return;  // no unstable cell in the tile
   local_ccl(lab, c.connectivity, gy0, gx0, c.nx, parent);
@@ -334,16 +447,7 @@ __global__ void __launch_bounds__(kThreads)
       const long long flat = (long long)r * c.nx + col;
       u = mask[flat] != 0;
       parent[flat] = u ? (int)flat : -1;
-      if (u) {
-        roots.count[flat] = 0;
-        roots.area6[flat] = 0;
-        roots.volume[flat] = 0;
-        roots.exc_start[flat] = 0;
-        roots.exc_stop[flat] = 0;
-        roots.max_exc_start[flat] = 0;
-        roots.max_exc_stop[flat] = 0;
-        roots.prev_overlap[flat] = 0;
-      }
+      if (u) label_clear_root(roots, flat);
     }
     lab[li] = u ? li : -1;
   }

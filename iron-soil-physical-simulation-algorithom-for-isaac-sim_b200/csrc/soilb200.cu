@@ -1269,6 +1269,7 @@ static LabelConst make_label_const(const sb_ctx* ctx, const sb_label_params* p) 
   c.release_latches = p->release_settled_latches ? 1 : 0;
   c.tile_size = ctx->d.tile_size;
   c.frontier_tiles_x = ctx->ftiles1;
+  c.yield = yield_constants(c);
   return c;
 }
 
@@ -1277,7 +1278,7 @@ static int run_label(sb_ctx* ctx, const LabelConst& c) {
   using T = FvTypes<FX>;
   const int tiles = c.tiles_x * ((c.ny + kLabelTile - 1) / kLabelTile);
   SB_CUDA(ctx, cudaMemsetAsync(ctx->lout, 0, sizeof(LabelOut), ctx->stream));
-  label_init_local_kernel<FX><<<tiles, kLabelInitThreads, 0, ctx->stream>>>(
+  label_init_local_kernel<FX><<<tiles, kLabelInitThreads<FX>, 0, ctx->stream>>>(
       c, (const typename T::B*)ctx->b, (const typename T::B*)ctx->z,
       (const typename T::H*)ctx->h[0], (const typename T::H*)ctx->h[1],
       (const typename T::R*)ctx->qx[0], (const typename T::R*)ctx->qx[1],
@@ -2290,7 +2291,7 @@ int build_path_graph(sb_ctx* ctx, const sb_path_params* p) {
                     &ctx->qy[0], &ctx->qy[1], &ctx->ctl, &ctx->parent, &ctx->slope, &ctx->severity,
                     &ctx->latch, &ctx->export_cum, &ctx->export_base, &ctx->roots};
     if ((rc = add_kernel(ctx, g, &node, &prev, 1, (void*)label_init_local_kernel<FX>, dim3(ltiles),
-                         0, args, kLabelInitThreads)))
+                         0, args, kLabelInitThreads<FX>)))
       return rc;
     prev = node;
   }

@@ -126,3 +126,29 @@ def test_yield_around_its_calm_line(start, stop, cohesion):
     assert np.array_equal(bridge.labels(), L.canonical_labels(want["unstable"], 8))
     assert np.array_equal(grid.download("severity").astype(np.float32), want["severity"])
     grid.close()
+
+
+@pytest.mark.parametrize("release", [False, True])
+@pytest.mark.parametrize("shape", [(2, 2), (3, 2), (33, 31), (31, 34), (64, 36), (40, 67)])
+def test_yield_quads_at_tile_and_row_edges(shape, release):
+    """Four cells per thread: widths that are and are not whole quads and tiles,
+    and a surface whose differences leave 32 bits (heights of +-2^31 quanta)."""
+    rng = np.random.default_rng(shape[0] * 100 + shape[1])
+    for scale in (0.05, 100.0):
+        b = scale * rng.uniform(-1.0, 1.0, shape)
+        z = b - 0.2 * rng.random(shape)
+        h = np.where(rng.random(shape) < 0.3, 0.1 * rng.random(shape), 0.0)
+        zero = np.zeros(shape)
+        grid = _grid(shape, b, z, h, zero, zero)
+        bridge = soilb200.B200LargeAvalancheBridge(
+            grid, soilb200.MaterialScenario("m", 1370.0, 29.8, 0.0, 0.5, 38.0, 30.0, 0.35))
+        bridge.label(release_settled_latches=release)
+        want = L.yield_init(fx.quantize(b, 0.0, K), fx.quantize(z, 0.0, K), fx.quantize(h, 0.0, K),
+                            None, None, dx=DX, dy=DY, tan_start=np.tan(np.deg2rad(38.0)),
+                            tan_stop=np.tan(np.deg2rad(30.0)), density=1370.0, gravity=9.81,
+                            cohesion=0.0, mobilization_depth=0.08, dry=1e-8, fixed_point=True,
+                            quantum=Q)
+        assert np.array_equal(bridge.labels(), L.canonical_labels(want["unstable"], 8))
+        for name in ("slope", "severity"):
+            assert np.array_equal(grid.download(name).astype(np.float32), want[name])
+        grid.close()
