@@ -15,8 +15,9 @@ bucket cut of the config; synthetic data, no dataset.
           the pinned-host -> device copy of the cut command (indices + target
           surfaces) and the device -> host read of the step records.
   roofline  dominant kernel = the fused FV substep kernel; achieved =
-          28 B/cell * cells per launch / mean launch time from CUDA events
-          recorded around the device-side substep loop.
+          28 B/cell * cells of the visited (not dry) blocks / mean time per
+          substep from CUDA events recorded around the device-side substep
+          loop.
 
 ``--impl reference`` times the CPU restatement of the reference path (NumPy,
 oracle/) on the same workload, one rank only.
@@ -163,19 +164,27 @@ class ClockSampler:
                 "samples": len(self.samples), "source": self.source}
 
 
+def visited_cells(h) -> int:
+    """Cells of the blocks (16 rows of a 30-column strip) that the substep loop
+    visits: those with mobile material in them or in a neighbour."""
+    rows, cols = -(-h.shape[0] // 16), -(-h.shape[1] // 30)
+    pad = np.zeros((rows * 16, cols * 30), dtype=bool)
+    pad[:h.shape[0], :h.shape[1]] = h > 0.0
+    wet = np.pad(pad.reshape(rows, 16, cols, 30).any(axis=(1, 3)), 1)
+    near = np.zeros((rows, cols), dtype=bool)
+    for dr in range(3):
+        for dc in range(3):
+            near |= wet[dr:dr + rows, dc:dc + cols]
+    return min(int(near.sum()) * 16 * 30, h.size)
+
+
 # DRAM bytes (read + write) per FV substep, from one ncu capture of the
 # persistent substep-loop kernel on the same workload (dram__bytes_read.sum +
 # dram__bytes_write.sum of the launch, divided by the substeps it ran).
 NCU_TRAFFIC_BYTES = {
-    # fv_loop_kernel at 701^2, 3 substeps in the captured launch: 8.028672 MB
-    # read + 1.536 KB written (cold L2 under ncu; the state then stays in L2)
-    "config1_plain_path_701": (8_028_672 + 1_536) // 3,
     # fv_loop_kernel at 4096^2, 4 substeps in the captured launch: 1.130031 GB
     # read + 805.078784 MB written
     "mobile_v2_4096": (1_130_031_000 + 805_078_784) // 4,
-    # fv_loop_kernel on the config-4 site (4096^2, 64 cuts), the first timed
-    # step's launch, 3 substeps: 841.548288 MB read + 592.439552 MB written
-    "site_c4_4096": (841_548_288 + 592_439_552) // 3,
 }
 
 
@@ -309,7 +318,8 @@ def run_gpu(args, rank: int, world: int, local_rank: int):
     tot_loop = sum(m for m, _ in loop_ms)
     tot_launch = sum(n for _, n in loop_ms)
     per_launch_ms = tot_loop / tot_launch if tot_launch else None
-    alg_bytes = BYTES_PER_CELL_SUBSTEP * cells
+    # dry blocks are neither read nor written: only the visited ones count
+    alg_bytes = BYTES_PER_CELL_SUBSTEP * visited_cells(h_fx)
     achieved = alg_bytes / (per_launch_ms * 1e-3) / 1e9 if per_launch_ms else None
     result = None
     if rank == 0:
@@ -342,10 +352,10 @@ def run_gpu(args, rank: int, world: int, local_rank: int):
                          "frac": (achieved / peak) if achieved else None,
                          "peak_source": peak_kind,
                          "algorithmic_bytes_per_launch": alg_bytes,
+                         "algorithmic_bytes": "28 B per cell of the blocks with mobile material "
+                                              "in or beside them in the final state",
                          "mean_launch_ms": per_launch_ms,
-                         "traffic": NCU_TRAFFIC_BYTES.get(args.workload),
-                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum "
-                                           "of one loop launch / its substeps"},
+                         "traffic": None},
             "gpu_launches": int(launches),
             "clocks": clocks.summary(),
             "wet_cells": wet_cells,
