@@ -17,7 +17,7 @@
 // barrier, and parities are compile-time because box origins are even.
 //
 // What bounds it: integer issue and instruction fetch (straight-line code; ncu
-// with 48 rows: 2.8 of 6.9 cycles per instruction wait for instructions).  A
+// with 48 rows in a box: 2.8 of 6.9 cycles per instruction wait for them).  A
 // pair is 8 integer operations (difference, clamp to +-C, excess, half of it
 // towards zero, the two new heights, the two running extremes); the
 // shared-memory kernel it replaces spent about 40 on index arithmetic, 64-bit
@@ -47,8 +47,12 @@ namespace sb {
 constexpr int kSweepHalo = 8;
 constexpr int kSweepCols = 64;                            // box columns of a warp
 constexpr int kSweepInner = kSweepCols - 2 * kSweepHalo;  // columns written back
-// Box rows; relax_full chooses.
-constexpr int kSweepRows = 24, kSweepRowsTall = 48;
+// Box rows.  Fixed point, measured per sweep, a cut pile settling / every box
+// moving (us): 701^2 20 rows 4.8 / 9.8, 24 rows 4.9 / 7.8, 28 rows 6.1 / 8.3, 32
+// rows 7.0 / 9.1, 48 rows 10.1 / 14.7; 2048^2 20 rows 11.4 / 47, 24 rows 9.2 / 32,
+// 28 rows 10.9 / 32, 32 rows 9.8 / 33.  More rows redo less halo, but the box's
+// straight-line code outgrows the instruction cache.
+constexpr int kSweepRows = 24;
 constexpr int kSweepThreads = 128;
 constexpr unsigned kSweepPolls = 1u << 22;
 
@@ -210,11 +214,13 @@ struct SweepOp<false, GEN> {
 // pairs have just been brought to the critical difference: never above it in
 // whole quanta, possibly by a rounding in FP64.  Once the tile is hot the
 // outcome of the test is known, so they are only looked at while it is not.
-template <bool FX, bool GEN, int R>
-__device__ __forceinline__ void sweep_box(const SweepConst& c, typename SweepOp<FX, GEN>::H (&e)[R],
-                                          typename SweepOp<FX, GEN>::H (&o)[R], int lane,
+template <bool FX, bool GEN>
+__device__ __forceinline__ void sweep_box(const SweepConst& c,
+                                          typename SweepOp<FX, GEN>::H (&e)[kSweepRows],
+                                          typename SweepOp<FX, GEN>::H (&o)[kSweepRows], int lane,
                                           bool okin, bool oknext, bool okprev, int rlo, int rhi,
                                           bool& hot, bool& chg) {
+  constexpr int R = kSweepRows;
   using S = SweepOp<FX, GEN>;
   using H = typename S::H;
   using L = typename S::L;
@@ -299,13 +305,13 @@ __device__ __forceinline__ void sweep_box(const SweepConst& c, typename SweepOp<
   chg = __any_sync(kAll, moved && lane >= 3 && lane < 29);
 }
 
-template <bool FX, int R>
-__global__ void __launch_bounds__(kSweepThreads, !FX ? 2 : R > 32 ? 3 : 4)
+template <bool FX>
+__global__ void __launch_bounds__(kSweepThreads, FX ? 4 : 2)
     sweep_kernel(const SweepConst c, typename FvTypes<FX>::H* f0, typename FvTypes<FX>::H* f1,
                  int* act0, int* act1, SweepControl* ctl) {
   using H = typename FvTypes<FX>::H;
   using H2 = typename std::conditional<FX, int2, double2>::type;
-  constexpr int kRows = R - 2 * kSweepHalo;
+  constexpr int R = kSweepRows, kRows = R - 2 * kSweepHalo;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // neighbouring tiles go to different SMs: active tiles come in clusters
   const int first = warp * gridDim.x + blockIdx.x, stride = gridDim.x * (kSweepThreads / 32);
@@ -364,9 +370,9 @@ __global__ void __launch_bounds__(kSweepThreads, !FX ? 2 : R > 32 ? 3 : 4)
       const bool okprev = oke && g1 > 0 && lane > 0;
       bool hot, chg;
       if (gen)
-        sweep_box<FX, true, R>(c, e, o, lane, okin, oknext, okprev, rlo, rhi, hot, chg);
+        sweep_box<FX, true>(c, e, o, lane, okin, oknext, okprev, rlo, rhi, hot, chg);
       else
-        sweep_box<FX, false, R>(c, e, o, lane, okin, oknext, okprev, rlo, rhi, hot, chg);
+        sweep_box<FX, false>(c, e, o, lane, okin, oknext, okprev, rlo, rhi, hot, chg);
       seen |= hot;
       if (lane == 0) next[t] = chg ? 1 : 0;
       // the other buffer already holds the interior if it moved neither in this

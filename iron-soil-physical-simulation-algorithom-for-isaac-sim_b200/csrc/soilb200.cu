@@ -1462,14 +1462,15 @@ __global__ void relax_reset_kernel(RelaxControl* ctl) {
 
 // Constants of a full-domain relaxation and its cooperative launch: every CTA
 // resident, at most one warp per tile.
-template <bool FX, int R>
+template <bool FX>
 static int launch_sweeps(sb_ctx* ctx, const RelaxConst& c) {
+  constexpr int inner = kSweepRows - 2 * kSweepHalo;  // rows written back
   SweepConst k{};
   k.n0 = c.n0;
   k.n1 = c.n1;
   k.pitch = c.pitch;
   k.tiles1 = (c.n1 + kSweepInner - 1) / kSweepInner;
-  k.ntiles = k.tiles1 * ((c.n0 + R - 2 * kSweepHalo - 1) / (R - 2 * kSweepHalo));
+  k.ntiles = k.tiles1 * ((c.n0 + inner - 1) / inner);
   k.max_iterations = c.max_iterations;
   k.tol = c.tol;
   for (int d = 0; d < 4; ++d) {
@@ -1486,14 +1487,14 @@ static int launch_sweeps(sb_ctx* ctx, const RelaxConst& c) {
   }
   const int per = kSweepThreads / 32;
   int ctas = 0;  // as many as fit the device at once
-  SB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, sweep_kernel<FX, R>,
+  SB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, sweep_kernel<FX>,
                                                              kSweepThreads, 0));
   const int grid = std::min((k.ntiles + per - 1) / per, std::max(1, ctas * ctx->sms));
   typename FvTypes<FX>::H *f0 = (typename FvTypes<FX>::H*)ctx->b,
                           *f1 = (typename FvTypes<FX>::H*)ctx->b_alt;
   int *a0 = ctx->sweep_act, *a1 = ctx->sweep_act + k.ntiles;
   void* args[] = {(void*)&k, (void*)&f0, (void*)&f1, (void*)&a0, (void*)&a1, (void*)&ctx->sweep};
-  SB_CUDA(ctx, cudaLaunchCooperativeKernel((void*)sweep_kernel<FX, R>, dim3(grid),
+  SB_CUDA(ctx, cudaLaunchCooperativeKernel((void*)sweep_kernel<FX>, dim3(grid),
                                            dim3(kSweepThreads), args, 0, ctx->stream));
   ctx->launches++;
   return SB_OK;
@@ -1503,21 +1504,7 @@ static int relax_full(sb_ctx* ctx, const sb_relax_params* p) {
   RelaxConst c;
   int rc = relax_const(ctx, p, &c, kRelaxTile);
   if (rc) return rc;
-  if (!fx(ctx)) return launch_sweeps<false, kSweepRows>(ctx, c);
-  // Box rows.  Measured per sweep, a cut pile settling / every box moving (us):
-  // 701^2 20 rows 4.8 / 9.8, 24 rows 4.9 / 7.8, 28 rows 6.1 / 8.3, 32 rows 7.0 /
-  // 9.1, 48 rows 10.1 / 14.7; 2048^2 20 rows 11.4 / 47, 24 rows 9.2 / 32, 28 rows
-  // 10.9 / 32, 32 rows 9.8 / 33.  More rows redo less halo, but the box's
-  // straight-line code outgrows the instruction cache.
-  // Grids of 2^18 .. 2^20 cells relax to the tolerance with 48 rows all the same
-  // (runs bounded to fewer than 64 iterations do not): there the learned schedule
-  // is required to take at most half the plain sweeps' time
-  // (tests/test_learned_gain_gpu.py), and a proposal's network does not get
-  // faster with the sweeps.
-  const long long cells = (long long)ctx->d.ny * ctx->d.nx;
-  if (c.max_iterations >= 64 && cells >= (1 << 18) && cells <= (1 << 20))
-    return launch_sweeps<true, kSweepRowsTall>(ctx, c);
-  return launch_sweeps<true, kSweepRows>(ctx, c);
+  return fx(ctx) ? launch_sweeps<true>(ctx, c) : launch_sweeps<false>(ctx, c);
 }
 
 // Queues max_iterations (or fewer, if converged) sweeps without waiting for

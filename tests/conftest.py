@@ -22,6 +22,12 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: requires a CUDA GPU (B200, sm_100a)")
 
 
+def pytest_collection_modifyitems(items):
+    """The comparison of two measured times comes last: under ``-x`` a miss of
+    its ratio must not hide the tests of results behind it."""
+    items.sort(key=lambda item: item.path.name == "test_learned_gain_gpu.py")
+
+
 @pytest.fixture(scope="session")
 def fv_golden():
     return np.load(GOLDEN / "fv_contracts.npz")
