@@ -157,17 +157,32 @@ struct ConvSmem {
 // Starts the copy of pixels [x, x + n) of an image row of C channels into a
 // staged row: 16-byte pieces, neighbouring threads on neighbouring addresses
 // (a thread per pixel instead asks L2 for every sector twice); zeros outside the
-// image and where row is false.
-template <int C, int NT>
+// image and where row is false.  ALIGNED = false: for images that do not start on 16
+// bytes, whose elements are copied one by one (a 16-byte copy would fault).
+template <int C, int NT, bool ALIGNED = true>
 __device__ __forceinline__ void row_async(const __nv_bfloat16* __restrict__ image, int w, bool row,
                                           int r, int x, int n, uint32_t dst) {
   const __nv_bfloat16* src = image + (size_t)(row ? r : 0) * w * C;
   for (int i = threadIdx.x; i < n * (C / 8); i += NT) {
     const int p = i / (C / 8), c8 = i % (C / 8);
     const bool ok = row && x + p >= 0 && x + p < w;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + c8 * kRowLbo + p * 16),
-                 "l"(src + (ok ? (size_t)(x + p) * C : 0) + c8 * 8), "r"(ok ? 16u : 0u)
-                 : "memory");
+    const __nv_bfloat16* from = src + (ok ? (size_t)(x + p) * C : 0) + c8 * 8;
+    const uint32_t to = dst + c8 * kRowLbo + p * 16;
+    if constexpr (ALIGNED) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from),
+                   "r"(ok ? 16u : 0u)
+                   : "memory");
+    } else {
+      uint32_t v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const unsigned short* e = reinterpret_cast<const unsigned short*>(from) + 2 * k;
+        v[k] = ok ? (uint32_t)e[0] | (uint32_t)e[1] << 16 : 0u;
+      }
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to), "r"(v[0]), "r"(v[1]),
+                   "r"(v[2]), "r"(v[3])
+                   : "memory");
+    }
   }
 }
 
@@ -630,7 +645,7 @@ struct WgradSmem {
 // accumulators (192 columns) and room for two CTAs per SM.  32 images of 128 x 128 x 32
 // (67 MB, 10 us at the copy rate): 31 to 40 us; one row per step and one CTA of two
 // bands per SM 57 to 61 us; rows transposed with 2-byte stores 147 to 186 us.
-template <int CIN, int COUT>
+template <int CIN, int COUT, bool ALIGNED>
 __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_tc_kernel(const WgradArgs a) {
   using S = WgradSmem<CIN, COUT>;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -650,11 +665,12 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_tc_kernel(const Wg
     const int y = y0 + 2 * i;
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      row_async<CIN, kConvThreads>(in, a.w, y - 1 + k >= 0 && y - 1 + k < a.h, y - 1 + k, x0 - 1, npx + 2,
-                           dst + k * S::ROW);
+      row_async<CIN, kConvThreads, ALIGNED>(in, a.w, y - 1 + k >= 0 && y - 1 + k < a.h, y - 1 + k,
+                                            x0 - 1, npx + 2, dst + k * S::ROW);
 #pragma unroll
     for (int k = 0; k < 2; ++k)
-      row_async<COUT, kConvThreads>(grad, a.w, y + k < y1, y + k, x0, npx, dst + 4 * S::ROW + k * S::G_ROW);
+      row_async<COUT, kConvThreads, ALIGNED>(grad, a.w, y + k < y1, y + k, x0, npx,
+                                             dst + 4 * S::ROW + k * S::G_ROW);
   };
   load(0);
   asm volatile("cp.async.commit_group;" ::: "memory");

@@ -38,21 +38,30 @@ cudaError_t launch_conv(const ConvArgs& a, int rows, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-template <int CIN, int COUT>
-cudaError_t launch_wgrad(const WgradArgs& a, cudaStream_t st) {
+template <int CIN, int COUT, bool ALIGNED>
+cudaError_t launch_wgrad_rows(const WgradArgs& a, cudaStream_t st) {
   using S = WgradSmem<CIN, COUT>;
   static bool attr_set[16] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 16 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(conv3x3_wgrad_tc_kernel<CIN, COUT>,
+    cudaError_t e = cudaFuncSetAttribute(conv3x3_wgrad_tc_kernel<CIN, COUT, ALIGNED>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES);
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  conv3x3_wgrad_tc_kernel<CIN, COUT>
+  conv3x3_wgrad_tc_kernel<CIN, COUT, ALIGNED>
       <<<a.tiles * a.chunks * a.batch, kConvThreads, S::BYTES, st>>>(a);
   return cudaGetLastError();
+}
+
+// Rows are copied in 16-byte pieces where both images start on 16 bytes (every
+// pixel then does), else element by element: tensors cut out of a larger buffer
+// are accepted wherever they start.
+template <int CIN, int COUT>
+cudaError_t launch_wgrad(const WgradArgs& a, cudaStream_t st) {
+  if (((uintptr_t)a.in | (uintptr_t)a.grad) & 15) return launch_wgrad_rows<CIN, COUT, false>(a, st);
+  return launch_wgrad_rows<CIN, COUT, true>(a, st);
 }
 
 bool conv_shape_ok(int cin, int cout) {
