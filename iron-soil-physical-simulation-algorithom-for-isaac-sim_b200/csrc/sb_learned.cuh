@@ -684,9 +684,14 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_tc_kernel(const Wg
   tc_fence_after();
   const uint32_t tmem = *tslot;
   const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-  const uint32_t idesc = umma_idesc_bf16(128, 2 * COUT, true);
+  // a band's last row without a partner is a step of its own columns alone (N =
+  // COUT): against the zeros in the partner's place an infinite input would leave a
+  // NaN in outputs that it has no part in
+  const uint32_t idesc_two = umma_idesc_bf16(128, 2 * COUT, true);
+  const uint32_t idesc_one = umma_idesc_bf16(128, COUT, true);
   bool ok = true;
   for (int i = 0; i < steps; ++i) {
+    const uint32_t idesc = y0 + 2 * i + 1 < y1 ? idesc_two : idesc_one;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     fence_async_smem();
     __syncthreads();  // step i's rows are staged
@@ -712,12 +717,13 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_wgrad_tc_kernel(const Wg
   tc_fence_after();
   __syncthreads();  // every MMA has completed: the stages' place takes the sums
   // warp = input row of the window, lane = ci.  Row s and output row j (0, 1) of the
-  // step are dy = s - j: first the shares of j = 0, then those of j = 1 on top.
+  // step are dy = s - j: first the shares of j = 0, then those of j = 1 on top (a band
+  // of one row has none).
   float* fold = reinterpret_cast<float*>(smem);
 #pragma unroll 1
   for (int j = 0; j < 2; ++j) {
     const int dy = warp - j;
-    if (dy >= 0 && dy < 3) {
+    if (dy >= 0 && dy < 3 && y0 + j < y1) {
 #pragma unroll 1
       for (int dx = 0; dx < 3; ++dx) {
         float v[COUT];
