@@ -317,15 +317,18 @@ class LearnedRelaxation:
         self.tan_crit = float(np.tan(np.deg2rad(critical_angle_deg)))
         ny, nx = grid.shape
         dev = net.device
-        self._feat = torch.empty(1, ny, nx, 16, dtype=torch.bfloat16, device=dev)
-        self._flux = torch.empty(ny * nx * 4, dtype=torch.float32, device=dev)
-        self._tq = torch.empty(ny * nx * 4, dtype=torch.int32, device=dev)
-        self._packed = net.packed()
         self._stream = grid.stream_handle()
-        # buffers made during a proposal belong to the grid's stream, so the
-        # allocator never hands them out while that stream still reads them
         self._torch_stream = torch.cuda.ExternalStream(self._stream, device=dev)
-        torch.cuda.current_stream(dev).synchronize()
+        # whatever a proposal reads or writes belongs to the grid's stream, so the
+        # allocator never hands it out while that stream still uses it (a queued
+        # proposal may outlive this object)
+        self._torch_stream.wait_stream(torch.cuda.current_stream(dev))  # the weights
+        with torch.cuda.stream(self._torch_stream):
+            self._feat = torch.empty(1, ny, nx, 16, dtype=torch.bfloat16, device=dev)
+            self._flux = torch.empty(ny * nx * 4, dtype=torch.float32, device=dev)
+            self._tq = torch.empty(ny * nx * 4, dtype=torch.int32, device=dev)
+            self._packed = net.packed()
+        self._torch_stream.synchronize()  # the weights may change from here on
 
     def propose(self, rounds: int = 1, scale: float = 1.0) -> None:
         """``rounds`` proposals; each moves ``scale`` times the network's
