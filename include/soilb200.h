@@ -241,8 +241,12 @@ typedef struct sb_relax_stats {
 int sb_relax_full(sb_ctx* ctx, const sb_relax_params* params, sb_relax_stats* out);
 /* The same sweeps queued on the context's stream without waiting for them or
  * reading statistics back (at most max_iterations; for interleaving with other
- * device work, e.g. learned proposals). */
+ * device work, e.g. learned proposals).  A wait of theirs that gave up is
+ * reported by the next sb_relax_full (SB_ERR_WAIT_LIMIT). */
 int sb_relax_sweeps(sb_ctx* ctx, const sb_relax_params* params);
+/* How often a CTA of a sweep polls for the others before it gives up (2^22 times
+ * at first, restored by a negative number). */
+int sb_relax_wait_polls(sb_ctx* ctx, int polls);
 /* Event-driven reached-bbox MiniSlope on SB_FIELD_B_EFF
  * (EventDrivenMinimumSlopeAdapter._relax_dynamic_frontier,
  * solvers/event_driven_slope.py:166-302): seeds = the current

@@ -59,6 +59,7 @@ constexpr unsigned kSweepPolls = 1u << 22;
 struct SweepConst {
   int n0, n1, pitch, tiles1, ntiles;
   int max_iterations;
+  unsigned polls;    // of a wait at the barrier
   double crit[4];    // FP64: critical difference per direction
   double tol;
   unsigned C[4];     // FX: largest difference in quanta that does not move
@@ -70,7 +71,7 @@ struct SweepControl {
   unsigned int leave;
   int iterations;
   int converged;
-  int status;
+  int status;  // 6: a wait gave up, in this or an earlier call; cleared by the host's report
 };
 
 // Arithmetic of one pair.  GEN = false: int32 differences (every height of the
@@ -317,7 +318,6 @@ __global__ void __launch_bounds__(kSweepThreads, FX ? 4 : 2)
   const int first = warp * gridDim.x + blockIdx.x, stride = gridDim.x * (kSweepThreads / 32);
   const int tiles0 = c.ntiles / c.tiles1;
   __shared__ int s_state;  // 0: next iteration, 1: converged, 2: stop, 3: a wait gave up
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->status = 0;
   int it = 0;
   for (;; ++it) {
     const H* src = (it & 1) ? f1 : f0;
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(kSweepThreads, FX ? 4 : 2)
       v += 1ull + ((unsigned long long)(any ? 1 : 0) << 32);
       unsigned polls = 0;
       while ((unsigned)v != gridDim.x) {
-        if (++polls > kSweepPolls) break;
+        if (++polls > c.polls) break;
         if (polls > 64) __nanosleep(32);
         v = *(volatile unsigned long long*)slot;
       }

@@ -204,6 +204,7 @@ struct sb_ctx {
   // full-domain sweeps: loop control, per-tile change flags (two iterations)
   SweepControl* sweep = nullptr;
   SweepControl* sweep_host = nullptr;
+  unsigned sweep_polls = kSweepPolls;
   int* sweep_act = nullptr;
   int sms = 1;
   LoopGraph relax_reached;  // reached-gated (event-driven) sweep to tolerance
@@ -1472,6 +1473,7 @@ static int launch_sweeps(sb_ctx* ctx, const RelaxConst& c) {
   k.tiles1 = (c.n1 + kSweepInner - 1) / kSweepInner;
   k.ntiles = k.tiles1 * ((c.n0 + inner - 1) / inner);
   k.max_iterations = c.max_iterations;
+  k.polls = ctx->sweep_polls;
   k.tol = c.tol;
   for (int d = 0; d < 4; ++d) {
     k.crit[d] = c.crit[d];
@@ -1507,6 +1509,12 @@ static int relax_full(sb_ctx* ctx, const sb_relax_params* p) {
   return fx(ctx) ? launch_sweeps<true>(ctx, c) : launch_sweeps<false>(ctx, c);
 }
 
+extern "C" int sb_relax_wait_polls(sb_ctx* ctx, int polls) {
+  if (!ctx) return SB_ERR_BAD_ARG;
+  ctx->sweep_polls = polls < 0 ? kSweepPolls : (unsigned)polls;
+  return SB_OK;
+}
+
 // Queues max_iterations (or fewer, if converged) sweeps without waiting for
 // them or reading their statistics back.
 extern "C" int sb_relax_sweeps(sb_ctx* ctx, const sb_relax_params* p) {
@@ -1526,8 +1534,11 @@ extern "C" int sb_relax_full(sb_ctx* ctx, const sb_relax_params* p, sb_relax_sta
   out->iterations = k.iterations;
   out->converged = k.converged;
   out->status = k.status;
-  if (k.status == SB_ERR_WAIT_LIMIT)
+  if (k.status == SB_ERR_WAIT_LIMIT) {
+    // of this call or of sweeps queued since the last report: reported once
+    SB_CUDA(ctx, cudaMemsetAsync(&ctx->sweep->status, 0, sizeof(int), ctx->stream));
     return fail(ctx, SB_ERR_WAIT_LIMIT, "[soilb200] a bounded device wait gave up (sweep barrier)");
+  }
   return SB_OK;
 }
 
