@@ -568,6 +568,12 @@ int sb_learned_propose(sb_ctx* ctx, void* feat, float* flux, int32_t* tq, const 
 int sb_last_error(sb_ctx* ctx, char* buffer, size_t length);
 /* Number of kernels this context has launched (cumulative). */
 int64_t sb_kernel_launch_count(sb_ctx* ctx);
+/* The blocks of which the fixed-point substep loop visits those with material in
+ * or beside them: rows of a chunk (chunks follow each other down the grid), rows
+ * of a chunk's blocks, columns; and how the last step's first substep took them:
+ * 0 shared out, 1 in runs (half of the grid is wet), 2 all (7/8).  Zeros where
+ * the loop does not run. */
+int sb_fv_blocks(sb_ctx* ctx, int out[4]);
 /* The cudaStream_t every operation of this context is issued on (for timing
  * with events or ordering caller work; do not destroy it). */
 void* sb_stream(sb_ctx* ctx);

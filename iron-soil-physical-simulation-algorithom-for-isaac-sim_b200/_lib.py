@@ -230,6 +230,7 @@ _PROTOTYPES = {
     "sb_mobile_ledger_of": (C.c_int, [C.c_void_p, C.POINTER(MobileParams),
                                       C.POINTER(MobileLedger)]),
     "sb_last_error": (C.c_int, [C.c_void_p, C.c_char_p, C.c_size_t]),
+    "sb_fv_blocks": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
     "sb_kernel_launch_count": (C.c_int64, [C.c_void_p]),
     "sb_stream": (C.c_void_p, [C.c_void_p]),
     "sb_version": (C.c_char_p, []),

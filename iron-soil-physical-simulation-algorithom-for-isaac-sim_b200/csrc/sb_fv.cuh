@@ -79,11 +79,10 @@ struct FvControl {
   // they left wet (high 32 bits); their total, for the substep's slot k % 3
   unsigned long long arrive_wet;
   int wetn[3];
-  // from the before-step ledger: its threads whose cells are mostly wet, and what
-  // that makes the first substep (LoopCtl.dense)
-  unsigned int wet_threads;
+  // from the before-step ledger: its threads that have cells, those whose cells are
+  // mostly wet, and what that makes the first substep (LoopCtl.dense)
+  unsigned int seen_threads, wet_threads;
   int dense;
-  int pad3;
 };
 
 // How the persistent loop visits its blocks when n of all are wet.  2 (at least

@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kThreads, FX ? kLedgerCtasFx : 3)
   __shared__ int last;
   double v[L_NP];
   long long iq[kLedgerI64] = {0, 0, 0};
-  bool mostly_wet = false;
+  bool seen = false, mostly_wet = false;  // a lane without a cell is neither wet nor dry
   const int nwarps = gridDim.x * (kThreads / 32);
   const int lane = threadIdx.x & 31;
   int it = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
@@ -467,7 +467,8 @@ __global__ void __launch_bounds__(kThreads, FX ? kLedgerCtasFx : 3)
                               col + lane * kLedgerQuad, scan);
     }
     scan.finish(c, v, iq);
-    mostly_wet = 2 * scan.wet_quads >= scan.quads;
+    seen = scan.quads > 0;
+    mostly_wet = seen && 2 * scan.wet_quads >= scan.quads;
   } else {
 #pragma unroll
     for (int k = 0; k < L_NP; ++k) v[k] = 0.0;
@@ -492,8 +493,16 @@ __global__ void __launch_bounds__(kThreads, FX ? kLedgerCtasFx : 3)
   double* part = mode == 0 ? part_before : partials;
   long long* ipart = mode == 0 ? ipart_before : ipartials;
   ledger_block_store(v, iq, fold, part + blockIdx.x, ipart + blockIdx.x, gridDim.x);
-  const int wet_threads = __syncthreads_count(mostly_wet);
-  if (FX && mode == 0 && threadIdx.x == 4) atomicAdd(&ctl->wet_threads, (unsigned)wet_threads);
+  if (FX && mode == 0) {
+    const int seen_threads = __syncthreads_count(seen);
+    const int wet_threads = __syncthreads_count(mostly_wet);
+    if (threadIdx.x == 4) {
+      atomicAdd(&ctl->seen_threads, (unsigned)seen_threads);
+      atomicAdd(&ctl->wet_threads, (unsigned)wet_threads);
+    }
+  } else {
+    __syncthreads();
+  }
   if (mode == 0 && threadIdx.x < 4) {  // the prologue's maxima (all >= 0: bits order like values)
     const int slot = threadIdx.x == 0 ? L_MAXEXT
                      : threadIdx.x == 1 ? L_MAXQ
@@ -519,7 +528,8 @@ __global__ void __launch_bounds__(kThreads, FX ? kLedgerCtasFx : 3)
       pro.v[L_MAXWAVE] = __longlong_as_double((long long)atomicExch(&ctl->pmax[3], 0ull));
       *arrive = 0;
       if (FX)
-        ctl->dense = fv_dense(atomicExch(&ctl->wet_threads, 0u), (long long)gridDim.x * kThreads);
+        ctl->dense =
+            fv_dense(atomicExch(&ctl->wet_threads, 0u), atomicExch(&ctl->seen_threads, 0u));
       ledger_prologue(c, &pro, static_limit, ctl);
       __threadfence();
       if (use_handle) cudaGraphSetConditional(loop_handle, ctl->done ? 0u : 1u);

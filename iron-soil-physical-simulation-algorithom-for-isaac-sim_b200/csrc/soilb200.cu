@@ -711,6 +711,16 @@ int sb_last_error(sb_ctx* ctx, char* buffer, size_t length) {
   return SB_OK;
 }
 
+int sb_fv_blocks(sb_ctx* ctx, int out[4]) {
+  if (!ctx || !out) return SB_ERR_BAD_ARG;
+  const bool loop = fx(ctx) && ctx->fv_stream && ctx->fv_persistent;
+  out[0] = loop ? ctx->fv_chunk_rows : 0;
+  out[1] = loop ? ctx->fv_block_rows : 0;
+  out[2] = loop ? kStripOut : 0;
+  out[3] = loop ? ctx->ctl_host->dense : 0;
+  return SB_OK;
+}
+
 int64_t sb_kernel_launch_count(sb_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
 void* sb_stream(sb_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }

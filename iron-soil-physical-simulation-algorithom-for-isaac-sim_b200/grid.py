@@ -148,6 +148,14 @@ class DeviceGrid:
     def synchronize(self) -> None:
         _lib.check(self.ctx, _lib.load().sb_synchronize(self.ctx), "synchronize")
 
+    def fv_blocks(self) -> tuple[int, int, int, int]:
+        """Rows of a chunk, rows and columns of a block of the fixed-point substep
+        loop, and how the last step's first substep took the blocks (0 shared out,
+        1 runs, 2 all)."""
+        out = (C.c_int * 4)()
+        _lib.check(self.ctx, _lib.load().sb_fv_blocks(self.ctx, out), "fv_blocks")
+        return tuple(out)
+
     def stream_handle(self) -> int:
         """Integer cudaStream_t of this context (e.g. for torch.cuda.ExternalStream)."""
         return int(_lib.load().sb_stream(self.ctx) or 0)
