@@ -164,18 +164,24 @@ class ClockSampler:
                 "samples": len(self.samples), "source": self.source}
 
 
-def visited_cells(h) -> int:
-    """Cells of the blocks (16 rows of a 30-column strip) that the substep loop
-    visits: those with mobile material in them or in a neighbour."""
-    rows, cols = -(-h.shape[0] // 16), -(-h.shape[1] // 30)
-    pad = np.zeros((rows * 16, cols * 30), dtype=bool)
-    pad[:h.shape[0], :h.shape[1]] = h > 0.0
-    wet = np.pad(pad.reshape(rows, 16, cols, 30).any(axis=(1, 3)), 1)
-    near = np.zeros((rows, cols), dtype=bool)
+def visited_cells(h, blocks) -> int:
+    """Cells of the blocks that the substep loop visits: those with mobile
+    material in them or in one of the eight blocks around.  ``blocks``: rows of a
+    chunk, rows and columns of a block (``DeviceGrid.fv_blocks``; a chunk's last
+    block may be shorter)."""
+    ny, nx = h.shape
+    chunk, height, width = blocks[:3]
+    if not chunk:  # no such loop: every cell
+        return h.size
+    tops = np.array([r for c in range(0, ny, chunk) for r in range(c, min(c + chunk, ny), height)])
+    lefts = np.arange(0, nx, width)
+    wet = np.logical_or.reduceat(np.logical_or.reduceat(h > 0.0, tops, axis=0), lefts, axis=1)
+    wet = np.pad(wet, 1)
+    near = np.zeros((tops.size, lefts.size), dtype=bool)
     for dr in range(3):
         for dc in range(3):
-            near |= wet[dr:dr + rows, dc:dc + cols]
-    return min(int(near.sum()) * 16 * 30, h.size)
+            near |= wet[dr:dr + tops.size, dc:dc + lefts.size]
+    return int(np.diff(tops, append=ny) @ near @ np.diff(lefts, append=nx))
 
 
 # DRAM bytes (read + write) per FV substep, from one ncu capture of the
@@ -319,7 +325,7 @@ def run_gpu(args, rank: int, world: int, local_rank: int):
     tot_launch = sum(n for _, n in loop_ms)
     per_launch_ms = tot_loop / tot_launch if tot_launch else None
     # dry blocks are neither read nor written: only the visited ones count
-    alg_bytes = BYTES_PER_CELL_SUBSTEP * visited_cells(h_fx)
+    alg_bytes = BYTES_PER_CELL_SUBSTEP * visited_cells(h_fx, grid.fv_blocks())
     achieved = alg_bytes / (per_launch_ms * 1e-3) / 1e9 if per_launch_ms else None
     result = None
     if rank == 0:
