@@ -56,7 +56,8 @@ struct YieldF {
   // A gradient below this is stable against both angles whatever the layer:
   // 1e-5 under the smaller tangent, where the margins' float32 rounding stays
   // below 1e-6 of the friction term; negative (never) for parameters of other
-  // signs.
+  // signs and for those so large or small that a term may overflow or lose its
+  // digits (the margins are then NaN, or rounding's).
   float calm;
 };
 
@@ -123,7 +124,8 @@ inline YieldF yield_constants(const LabelConst& c) {
   y.tp = (float)c.tan_stop;
   y.dts = (float)(c.tan_start - c.tan_stop);
   y.dry = (float)c.dry;
-  y.calm = y.coh >= 0.f && y.rg > 0.f && y.ts > 0.f && y.tp > 0.f && y.depth > 0.f
+  y.calm = y.coh >= 0.f && y.rg >= 1.0e-15f && y.rg <= 1.0e20f && y.ts > 0.f && y.ts <= 1.0e4f &&
+                   y.tp > 0.f && y.tp <= 1.0e4f && y.depth > 0.f
                ? std::fmin(y.ts, y.tp) * (1.f - 1.0e-5f)
                : -1.f;
   return y;
