@@ -317,18 +317,25 @@ class LearnedRelaxation:
         self.tan_crit = float(np.tan(np.deg2rad(critical_angle_deg)))
         ny, nx = grid.shape
         dev = net.device
+        self._feat = torch.empty(1, ny, nx, 16, dtype=torch.bfloat16, device=dev)
+        self._flux = torch.empty(ny * nx * 4, dtype=torch.float32, device=dev)
+        self._tq = torch.empty(ny * nx * 4, dtype=torch.int32, device=dev)
+        self._packed = net.packed()
         self._stream = grid.stream_handle()
+        # buffers made during a proposal belong to the grid's stream, so the
+        # allocator never hands them out while that stream still reads them; those
+        # above come from the caller's stream (whose cached blocks they reuse: on
+        # the grid's, a new object takes 1 to 3 ms more), so nothing may still run
+        # in them now, nor when they go (__del__)
         self._torch_stream = torch.cuda.ExternalStream(self._stream, device=dev)
-        # whatever a proposal reads or writes belongs to the grid's stream, so the
-        # allocator never hands it out while that stream still uses it (a queued
-        # proposal may outlive this object)
-        self._torch_stream.wait_stream(torch.cuda.current_stream(dev))  # the weights
-        with torch.cuda.stream(self._torch_stream):
-            self._feat = torch.empty(1, ny, nx, 16, dtype=torch.bfloat16, device=dev)
-            self._flux = torch.empty(ny * nx * 4, dtype=torch.float32, device=dev)
-            self._tq = torch.empty(ny * nx * 4, dtype=torch.int32, device=dev)
-            self._packed = net.packed()
-        self._torch_stream.synchronize()  # the weights may change from here on
+        torch.cuda.current_stream(dev).synchronize()
+
+    def __del__(self):
+        try:  # a closed grid has waited for its stream
+            if self.grid._ctx is not None:
+                self.grid.synchronize()
+        except Exception:  # half-made object, interpreter shutdown
+            pass
 
     def propose(self, rounds: int = 1, scale: float = 1.0) -> None:
         """``rounds`` proposals; each moves ``scale`` times the network's

@@ -1,6 +1,6 @@
-"""A proposal is queued on the grid's stream and may still run when the object
-that queued it is gone: its buffers belong to that stream, so that the allocator
-does not give them to work of another stream meanwhile."""
+"""A proposal is queued on the grid's stream and returns at once.  Dropping the
+object that queued it frees the proposal's buffers to other streams, so the drop
+waits for it."""
 
 import numpy as np
 import pytest
@@ -12,22 +12,28 @@ from soilb200 import learned
 pytestmark = pytest.mark.gpu
 
 
-def _stream_of(tensor) -> int:
-    p = tensor.data_ptr()
-    for seg in torch.cuda.memory_snapshot():
-        if seg["address"] <= p < seg["address"] + seg["total_size"]:
-            return int(seg["stream"])
-    raise AssertionError("not the allocator's memory")
-
-
 @pytest.mark.parametrize("fused", [True, False])
-def test_buffers_belong_to_the_grids_stream(fused):
-    grid = soilb200.DeviceGrid((70, 90), 0.05, 0.05, precision="fx32", height_exponent=28)
+def test_dropping_the_object_waits_for_its_proposals(fused):
+    shape = (1500, 1500)  # a round takes about 150 us, the drop some microseconds
+    grid = soilb200.DeviceGrid(shape, 0.05, 0.05, precision="fx32", height_exponent=28)
+    grid.upload("b_eff", np.random.default_rng(3).random(shape))
     lr = learned.LearnedRelaxation(grid, learned.ReposeNet(seed=1), 35.0, fused=fused)
-    held = [v for k, v in vars(lr).items() if isinstance(v, torch.Tensor)] + list(lr._packed)
-    assert len(held) >= 6
-    assert {_stream_of(t) for t in held} == {grid.stream_handle()}
+    stream = torch.cuda.ExternalStream(grid.stream_handle())
+    lr.propose(2)
+    grid.synchronize()
+    lr.propose(40)
+    del lr
+    assert stream.query()
     grid.close()
+
+
+def test_the_grid_may_close_first():
+    grid = soilb200.DeviceGrid((70, 90), 0.05, 0.05, precision="fx32", height_exponent=28)
+    lr = learned.LearnedRelaxation(grid, learned.ReposeNet(seed=1), 35.0)
+    lr.propose(3)
+    grid.close()
+    del lr
+    torch.cuda.synchronize()
 
 
 def test_weights_are_those_of_the_making():
