@@ -188,9 +188,15 @@ def visited_cells(h, blocks) -> int:
 # persistent substep-loop kernel on the same workload (dram__bytes_read.sum +
 # dram__bytes_write.sum of the launch, divided by the substeps it ran).
 NCU_TRAFFIC_BYTES = {
-    # fv_loop_kernel at 4096^2, 4 substeps in the captured launch: 1.130031 GB
-    # read + 805.078784 MB written
-    "mobile_v2_4096": (1_130_031_000 + 805_078_784) // 4,
+    # fv_loop_kernel at 701^2, 3 substeps in the captured launch: 277.248 KB read,
+    # nothing written (the visited blocks stay in L2 after their first touch)
+    "config1_plain_path_701": 277_248 // 3,
+    # fv_loop_kernel at 4096^2, 4 substeps in the captured launch: 1.109262 GB
+    # read + 789.439744 MB written
+    "mobile_v2_4096": (1_109_261_568 + 789_439_744) // 4,
+    # fv_loop_kernel on the config-4 site (4096^2, 64 cuts), the first timed
+    # step's launch, 3 substeps: 13.356544 MB read + 126.976 KB written
+    "site_c4_4096": (13_356_544 + 126_976) // 3,
 }
 
 
@@ -361,7 +367,9 @@ def run_gpu(args, rank: int, world: int, local_rank: int):
                          "algorithmic_bytes": "28 B per cell of the blocks with mobile material "
                                               "in or beside them in the final state",
                          "mean_launch_ms": per_launch_ms,
-                         "traffic": None},
+                         "traffic": NCU_TRAFFIC_BYTES.get(args.workload),
+                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum "
+                                           "of one loop launch / its substeps"},
             "gpu_launches": int(launches),
             "clocks": clocks.summary(),
             "wet_cells": wet_cells,
