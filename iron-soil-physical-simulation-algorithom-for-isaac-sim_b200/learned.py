@@ -347,12 +347,13 @@ class LearnedRelaxation:
             raise ValueError("[soilb200] the proposal scale must be positive")
         if self.fused:
             w = [p.data_ptr() for p in self._packed]
-            for _ in range(rounds):
-                # the transfer is flux * tan * dx, so the scale rides on tan
-                _lib.check(self.grid.ctx, lib.sb_learned_propose(
-                    self.grid.ctx, self._feat.data_ptr(), self._flux.data_ptr(),
-                    self._tq.data_ptr(), *w, self.tan_crit, self.tan_crit * scale,
-                    self.net.status.data_ptr()), "propose")
+            with torch.cuda.device(self.net.device):  # whichever is current at the call
+                for _ in range(rounds):
+                    # the transfer is flux * tan * dx, so the scale rides on tan
+                    _lib.check(self.grid.ctx, lib.sb_learned_propose(
+                        self.grid.ctx, self._feat.data_ptr(), self._flux.data_ptr(),
+                        self._tq.data_ptr(), *w, self.tan_crit, self.tan_crit * scale,
+                        self.net.status.data_ptr()), "propose")
             return
         with torch.cuda.stream(self._torch_stream):
             for _ in range(rounds):
