@@ -341,19 +341,23 @@ class LearnedRelaxation:
         """``rounds`` proposals; each moves ``scale`` times the network's
         transfer (flux * tan_crit * dx * scale per edge, still limited to half
         the height difference and rounded toward zero to whole quanta)."""
+        with _torch().cuda.device(self.net.device):
+            self._propose(rounds, scale)
+
+    def _propose(self, rounds: int, scale: float) -> None:
+        """On the grid's device: a launch on its stream fails with another current."""
         torch = _torch()
         lib = _lib.load()
         if not scale > 0.0:
             raise ValueError("[soilb200] the proposal scale must be positive")
         if self.fused:
             w = [p.data_ptr() for p in self._packed]
-            with torch.cuda.device(self.net.device):  # whichever is current at the call
-                for _ in range(rounds):
-                    # the transfer is flux * tan * dx, so the scale rides on tan
-                    _lib.check(self.grid.ctx, lib.sb_learned_propose(
-                        self.grid.ctx, self._feat.data_ptr(), self._flux.data_ptr(),
-                        self._tq.data_ptr(), *w, self.tan_crit, self.tan_crit * scale,
-                        self.net.status.data_ptr()), "propose")
+            for _ in range(rounds):
+                # the transfer is flux * tan * dx, so the scale rides on tan
+                _lib.check(self.grid.ctx, lib.sb_learned_propose(
+                    self.grid.ctx, self._feat.data_ptr(), self._flux.data_ptr(),
+                    self._tq.data_ptr(), *w, self.tan_crit, self.tan_crit * scale,
+                    self.net.status.data_ptr()), "propose")
             return
         with torch.cuda.stream(self._torch_stream):
             for _ in range(rounds):
@@ -408,26 +412,27 @@ class LearnedRelaxation:
             _lib.check(self.grid.ctx, lib.sb_relax_full(self.grid.ctx, p, st), "relax")
             return st
 
-        done = 0
-        for sc in scales:
-            self.propose(1, sc)
-            if plain_between > 0:
-                sweeps(plain_between)
-                done += plain_between
-        if check_sweeps > 0 and extra:
-            st = full(check_sweeps)
-            done += int(st.iterations)
-            if st.converged:
-                st.iterations = done
-                return st
-            for sc in extra:
-                self.propose(1, sc)
-                if extra_between > 0:
-                    sweeps(extra_between)
-                    done += extra_between
-        st = full(max_iterations)
-        st.iterations = int(st.iterations) + done
-        return st
+        with _torch().cuda.device(self.net.device):
+            done = 0
+            for sc in scales:
+                self._propose(1, sc)
+                if plain_between > 0:
+                    sweeps(plain_between)
+                    done += plain_between
+            if check_sweeps > 0 and extra:
+                st = full(check_sweeps)
+                done += int(st.iterations)
+                if st.converged:
+                    st.iterations = done
+                    return st
+                for sc in extra:
+                    self._propose(1, sc)
+                    if extra_between > 0:
+                        sweeps(extra_between)
+                        done += extra_between
+            st = full(max_iterations)
+            st.iterations = int(st.iterations) + done
+            return st
 
     def relax_scheduled(self, tolerance_m: float, schedule=None, max_iterations: int = 400000,
                         spacing=None):

@@ -1,5 +1,5 @@
-"""A proposal's kernels go to the grid's stream, so the grid's device has to be the
-current one at each of its calls, whichever it was before (a second GPU's grid in a
+"""Proposals and sweeps go to the grid's stream, so the grid's device has to be the
+current one at each of their calls, whichever it was before (a second GPU's grid in a
 process that works on the first).  On fakes of torch and of the library."""
 
 import contextlib
@@ -27,7 +27,8 @@ def test_proposals_run_on_the_grids_device(monkeypatch, fused):
     fake = SimpleNamespace(cuda=SimpleNamespace(device=device, stream=lambda s: device(s.device)))
     monkeypatch.setattr(learned, "_torch", lambda: fake)
     monkeypatch.setattr(learned._lib, "load", lambda: SimpleNamespace(
-        sb_learned_propose=call, sb_learned_features=call, sb_learned_apply=call))
+        sb_learned_propose=call, sb_learned_features=call, sb_learned_apply=call,
+        sb_relax_sweeps=call, sb_relax_full=call))
     buffer = SimpleNamespace(data_ptr=lambda: 0)
     monkeypatch.setattr(learned, "network_forward", lambda *a, **k: (call(), buffer))
     lr = object.__new__(learned.LearnedRelaxation)
@@ -39,4 +40,6 @@ def test_proposals_run_on_the_grids_device(monkeypatch, fused):
     lr._torch_stream = SimpleNamespace(device=1)
     lr.propose(3)
     assert seen == [1] * (3 if fused else 9)
+    lr.relax(1e-4, scales=(1.0, 0.5), rounds=2, plain_between=5, spacing=(0.05, 0.05))
+    assert seen == [1] * (3 + 5 if fused else 9 + 9)  # two rounds, two sweep calls, the last
     assert current == [0]
